@@ -318,6 +318,7 @@ SIGNATURES = {
     "tlm_slab_flush": (_st, [_h]),
     "tlm_get_halo_stream": (_st, [_h, _P(C.c_void_p)]),
     "tlm_step_launches": (_st, [_h, _P(C.c_int)]),
+    "tlm_steps_per_pass": (_st, [_h, _P(C.c_int)]),
     "tlm_near_field_box": (_st, [_h, _P(C.c_int)]),
 }
 

@@ -6,6 +6,7 @@
 #include "tlm_device.cuh"
 
 #include <atomic>
+#include <memory>
 #include <type_traits>
 #include <string>
 #include <vector>
@@ -181,6 +182,13 @@ struct SurfaceState
     void *dFrames = nullptr;
     size_t framesCap = 0, framesUsed = 0;  // elements
 };
+
+// The plan of two-step passes (tlm_pair_kernel.cuh; defined in tlm_solver.cu).
+struct PairPlan;
+
+// Two-step passes serve FP32 grids from this many padded nodes on.
+constexpr long long kPairMinNodes = 1LL << 20;
+inline bool pairStorage(int storage, long long P) { return storage == TLM_STORE_F32 && P >= kPairMinNodes; }
 } // namespace tlmi
 
 struct tlm_solver
@@ -273,6 +281,13 @@ struct tlm_solver
     bool slabBegun = false, slabOpen = false;
     int slabPos = 0;
     long long slabBase = 0, slabEFirst = 0;
+    // two steps per pass over memory: the plan, made on the first use after
+    // prepare (pairTried), its column flags, and the stub planes the next
+    // pass writes (swapped with dStub after every pass)
+    std::shared_ptr<tlmi::PairPlan> pair;
+    bool pairTried = false;
+    unsigned *dPairFlags = nullptr;
+    void *dStubAlt = nullptr;
     std::vector<uint8_t> tileFlagsHost;
     void *dSamples = nullptr;
     double *dEpart = nullptr;
@@ -299,6 +314,7 @@ struct tlm_solver
     bool timing = false;
     std::vector<cudaEvent_t> evs;
     size_t evUsed = 0;
+    long long timedSteps = 0;
 
     tlm_status fail(tlm_status s, const std::string &m)
     {

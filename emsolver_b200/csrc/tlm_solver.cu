@@ -8,6 +8,7 @@
 
 #include "tlm_aux_kernels.cuh"
 #include "tlm_host_math.h"
+#include "tlm_pair_kernel.cuh"
 #include "tlm_step_kernel.cuh"
 
 #include <algorithm>
@@ -17,6 +18,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <type_traits>
 #include <vector>
 
@@ -65,6 +67,10 @@ void freeMonitors(tlm_solver *h)
     devFree(h, h->dStaged);
     devFree(h, h->dListed);
     h->nStaged = h->nListed = 0;
+    h->pair.reset();
+    h->pairTried = false;
+    devFree(h, h->dPairFlags);
+    devFree(h, h->dStubAlt);
     devFree(h, h->dSamples);
     devFree(h, h->dEpart);
     devFree(h, h->dPortOff);
@@ -619,23 +625,30 @@ template <class S> tlmk::StepArgs<S> stepArgs(const tlm_solver *h, int n, int i,
     return a;
 }
 
+// Kernel timing: record the event before a launch that runs `steps` steps;
+// *after is the one to record behind it (null without timing).
+tlm_status timeLaunch(tlm_solver *h, int steps, cudaEvent_t *after)
+{
+    *after = nullptr;
+    if (!h->timing) return TLM_OK;
+    while (h->evs.size() < h->evUsed + 2)
+    {
+        cudaEvent_t ev;
+        TLM_CU(h, cudaEventCreate(&ev));
+        h->evs.push_back(ev);
+    }
+    *after = h->evs[h->evUsed + 1];
+    TLM_CU(h, cudaEventRecord(h->evs[h->evUsed], h->stream));
+    h->evUsed += 2;
+    h->timedSteps += steps;
+    return TLM_OK;
+}
+
 template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long eFirst)
 {
     const tlmk::StepArgs<S> a = stepArgs<S>(h, n, i, eFirst);
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (h->timing)
-    {
-        while (h->evs.size() < h->evUsed + 2)
-        {
-            cudaEvent_t ev;
-            TLM_CU(h, cudaEventCreate(&ev));
-            h->evs.push_back(ev);
-        }
-        e0 = h->evs[h->evUsed];
-        e1 = h->evs[h->evUsed + 1];
-        h->evUsed += 2;
-        TLM_CU(h, cudaEventRecord(e0, h->stream));
-    }
+    cudaEvent_t e1 = nullptr;
+    TLM_TRY(timeLaunch(h, 1, &e1));
     if (surfaceActive(h)) TLM_TRY(launchSurface(h, n));  // reads the same input buffer, first
     if constexpr (std::is_same<S, float>::value)
     {
@@ -685,8 +698,213 @@ template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long 
     else
         launchShaped<S>(a, h->variant, h->stateIncident, h->nblocks, h->stream);
     TLM_CU(h, cudaGetLastError());
-    if (h->timing) TLM_CU(h, cudaEventRecord(e1, h->stream));
+    if (e1) TLM_CU(h, cudaEventRecord(e1, h->stream));
     h->stateIncident = false;
+    h->curBuf ^= 1;
+    return TLM_OK;
+}
+
+// The kernel shapes of two-step passes: wide columns first (they measured 4 %
+// faster per plane than the second's where both fit a grid equally), then
+// taller ones, which leave fewer lanes idle on grids the first cuts badly.
+using PairLayouts = std::tuple<tlmk::PairLayout<50, 10, 3, 1>, tlmk::PairLayout<34, 15, 3, 1>>;
+template <int I = 0, class F> void withPairLayout(int layout, F &&f)
+{
+    if constexpr (I < (int)std::tuple_size<PairLayouts>::value)
+    {
+        if (layout == I)
+            f(std::tuple_element_t<I, PairLayouts>{});
+        else
+            withPairLayout<I + 1>(layout, f);
+    }
+}
+
+// The columns with the least cost: blocks run one per SM and every plane of
+// one costs about the same, so a pass takes waves x planes per block (two of
+// them first-step planes of the neighbouring ranges).
+void choosePairShape(int ny, int nz, int px, int sms, tlmk::PairShape &best, int &layout)
+{
+    long long bestCost = -1;
+    for (int l = 0; l < (int)std::tuple_size<PairLayouts>::value; ++l)
+        withPairLayout(l, [&](auto L) {
+            using Layout = decltype(L);
+            const int ntx = (px + Layout::maxTX - 1) / Layout::maxTX;
+            const int TX = ((px + ntx - 1) / ntx + 3) / 4 * 4;
+            const int nty0 = (ny + Layout::maxTY - 1) / Layout::maxTY;
+            for (int rows = nty0; rows < nty0 + 6 && rows <= ny; ++rows)
+            {
+                const int TY = (ny + rows - 1) / rows, nty = (ny + TY - 1) / TY;
+                for (int c = 1; c <= std::max(1, nz / 4); ++c)
+                {
+                    const long long waves = ((long long)ntx * nty * c + sms - 1) / sms;
+                    const long long cost = waves * ((nz + c - 1) / c + (c > 2 ? 2 : c - 1) + 1);
+                    if (bestCost >= 0 && cost >= bestCost) continue;
+                    bestCost = cost;
+                    best = tlmk::PairShape{ TX, TY, ntx, nty, c };
+                    layout = l;
+                }
+            }
+        });
+}
+
+} // namespace tlmi
+
+struct tlmi::PairPlan
+{
+    tlmk::PairShape sh{};
+    int layout = 0;
+    CUtensorMap map[2][3];  // per pulse buffer: boxes of x, y and z slots
+};
+
+namespace tlmi {
+
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiled encodeTiled()
+{
+    static EncodeTiled fn = []() -> EncodeTiled {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+        {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return reinterpret_cast<EncodeTiled>(p);
+    }();
+    return fn;
+}
+
+// Plan the two-step passes of a handle, once per prepare; without one (not
+// enough memory for the second set of stub planes, no tensor maps) the handle
+// keeps stepping one step per launch.
+tlm_status ensurePair(tlm_solver *h)
+{
+    if (h->pairTried) return TLM_OK;
+    h->pairTried = true;
+    EncodeTiled encode = encodeTiled();
+    if (!encode) return TLM_OK;
+    if (h->dStub)
+    {
+        const size_t need = 3 * (size_t)h->P * sizeof(float);
+        if (!poolCovers(h->device, need) && poolAvailable(h->device) < need + ((size_t)256 << 20)) return TLM_OK;
+    }
+    int sms = 0;
+    TLM_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    auto plan = std::make_shared<PairPlan>();
+    choosePairShape(h->ny, h->nz, h->px, sms, plan->sh, plan->layout);
+    const tlmk::PairShape &g = plan->sh;
+    // the kernel's lane offsets within a plane are 32-bit byte offsets, and
+    // its energy partials take the single-step kernels' places
+    if ((long long)h->px * h->ny > (1LL << 28) || (long long)g.ntx * g.nty * g.nchunk > h->nblocks) return TLM_OK;
+    tlm_status st = TLM_OK;
+    bool ok = true;
+    withPairLayout(plan->layout, [&](auto L) {
+        using Layout = decltype(L);
+        for (int b = 0; b < 2; ++b)
+            for (int m = 0; m < 3; ++m)
+            {
+                const cuuint64_t dims[4] = { (cuuint64_t)h->px, (cuuint64_t)h->ny, (cuuint64_t)h->nz, 12 };
+                const cuuint64_t strides[3] = { (cuuint64_t)h->px * 4, (cuuint64_t)h->px * h->ny * 4,
+                                                (cuuint64_t)h->P * 4 };
+                const cuuint32_t box[4] = { (cuuint32_t)Layout::W2, (cuuint32_t)(m == 1 ? Layout::H + 1 : Layout::H), 1,
+                                            m == 0 ? 4u : 2u };
+                const cuuint32_t es[4] = { 1, 1, 1, 1 };
+                ok = ok && encode(&plan->map[b][m], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->dPulses[b], dims, strides,
+                                  box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+            }
+        st = h->cuda(cudaFuncSetAttribute(tlmk::stepPairKernel<Layout, true>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, Layout::smemBytes),
+                     "cudaFuncSetAttribute(stepPairKernel)");
+        if (st == TLM_OK)
+            st = h->cuda(cudaFuncSetAttribute(tlmk::stepPairKernel<Layout, false>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, Layout::smemBytes),
+                         "cudaFuncSetAttribute(stepPairKernel)");
+    });
+    TLM_TRY(st);
+    if (!ok) return TLM_OK;
+    if (h->dStub)
+    {
+        if (devAlloc(h, &h->dStubAlt, 3 * (size_t)h->P * sizeof(float)) != TLM_OK) return TLM_OK;
+        TLM_CU(h, cudaMemsetAsync(h->dStubAlt, 0, 3 * (size_t)h->P * sizeof(float), h->stream));
+    }
+    const size_t nf = (size_t)g.ntx * g.nty * h->nz;
+    TLM_TRY(devAlloc(h, &h->dPairFlags, nf * sizeof(unsigned)));
+    TLM_CU(h, cudaMemsetAsync(h->dPairFlags, 0, nf * sizeof(unsigned), h->stream));
+    tlmk::pairMaterialFlags<<<(unsigned)nf, 128, 0, h->stream>>>(h->dMat, h->nx, h->ny, h->nz, h->px, g, h->dPairFlags);
+    if (h->specCount)
+        tlmk::pairSpecFlags<<<(h->specCount + 127) / 128, 128, 0, h->stream>>>(h->dSpec, h->specCount, h->ny, h->nz,
+                                                                               h->px, g, h->dPairFlags);
+    TLM_CU(h, cudaGetLastError());
+    h->pair = std::move(plan);
+    return TLM_OK;
+}
+
+// Whether the next two steps may share a pass: FP32 in the default shape,
+// nothing that reads the state between them (surface monitors) or splits the
+// step (slabs), reflected input.
+bool pairAllowed(const tlm_solver *h)
+{
+    return pairStorage(h->storage, h->P) && h->variant == 0 && !h->cfg.no_staging && !h->cfg.general_tiles &&
+           !h->ghostLo && !h->ghostHi && !surfaceActive(h) && !h->stateIncident;
+}
+
+// Steps n and n+1, the i-th and (i+1)-th of the window, in one pass.
+tlm_status launchPair(tlm_solver *h, int n, int i, long long eFirst)
+{
+    const PairPlan &pl = *h->pair;
+    const tlmk::StepArgs<float> s0 = stepArgs<float>(h, n, i, eFirst), s1 = stepArgs<float>(h, n + 1, i + 1, eFirst);
+    tlmk::PairArgs a;
+    a.mapX = pl.map[h->curBuf][0];
+    a.mapY = pl.map[h->curBuf][1];
+    a.mapZ = pl.map[h->curBuf][2];
+    a.sh = pl.sh;
+    a.in = s0.in;
+    a.out = s0.out;
+    a.stubIn = static_cast<const float *>(h->dStub);
+    a.stubOut = static_cast<float *>(h->dStubAlt);
+    a.mat = s0.mat;
+    a.yhat = s0.yhat;
+    a.ghat = s0.ghat;
+    a.ntable = (int)h->epsr.size();
+    a.flags = h->dPairFlags;
+    a.P = h->P;
+    a.nx = h->nx;
+    a.ny = h->ny;
+    a.nz = h->nz;
+    a.px = h->px;
+    a.rho = s0.rho;
+    a.spec = h->dSpec;
+    a.nspec = h->specCount;
+    a.sv[0] = s0.sv;
+    a.sv[1] = s1.sv;
+    a.samples[0] = s0.samples;
+    a.samples[1] = s1.samples;
+    a.epart[0] = s0.epart;
+    a.epart[1] = s1.epart;
+    a.nepart = h->nblocks;
+    a.neg_zero = -0.0f;
+    a.stage_wait_ns = s0.stage_wait_ns;
+    a.fault = h->dFault;
+    cudaEvent_t after = nullptr;
+    TLM_TRY(timeLaunch(h, 2, &after));
+    withPairLayout(pl.layout, [&](auto L) {
+        using Layout = decltype(L);
+        const unsigned blocks = (unsigned)(pl.sh.ntx * pl.sh.nty * pl.sh.nchunk);
+        if (h->dStub)
+            tlmk::stepPairKernel<Layout, true><<<blocks, Layout::kThreads, Layout::smemBytes, h->stream>>>(a);
+        else
+            tlmk::stepPairKernel<Layout, false><<<blocks, Layout::kThreads, Layout::smemBytes, h->stream>>>(a);
+    });
+    TLM_CU(h, cudaGetLastError());
+    if (after) TLM_CU(h, cudaEventRecord(after, h->stream));
+    if (h->dStubAlt) std::swap(h->dStub, h->dStubAlt);
     h->curBuf ^= 1;
     return TLM_OK;
 }
@@ -746,6 +964,16 @@ tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stoppe
         for (int i = 0; i < w; ++i)
         {
             const int n = (int)(base + i);
+            if (i + 1 < w && pairAllowed(h))
+            {
+                TLM_TRY(ensurePair(h));
+                if (h->pair)
+                {
+                    TLM_TRY(launchPair(h, n, i, eFirst));
+                    ++i;
+                    continue;
+                }
+            }
             switch (h->storage)
             {
             case TLM_STORE_F64: TLM_TRY(launchStep<double>(h, n, i, eFirst)); break;
@@ -1298,6 +1526,7 @@ tlm_status tlm_setup(tlm_handle h, const tlm_grid *grid, const uint8_t *mat, siz
     h->finished.store(false);
     h->stopFlag.store(false);
     h->evUsed = 0;
+    h->timedSteps = 0;
     h->scale = 1.0f;
     h->surf.planeAxis = -1;
     h->surf.planeIndex = 0;
@@ -2182,6 +2411,7 @@ tlm_status tlm_set_kernel_timing(tlm_handle h, int enable)
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->timing = enable != 0;
     h->evUsed = 0;
+    h->timedSteps = 0;
     return TLM_OK;
 }
 
@@ -2204,6 +2434,21 @@ tlm_status tlm_step_launches(tlm_handle h, int *per_step)
     return TLM_OK;
 }
 
+tlm_status tlm_steps_per_pass(tlm_handle h, int *steps)
+{
+    TLM_TRY(checkReady(h));
+    if (!steps) return h->fail(TLM_EINVAL, "null output");
+    DeviceGuard dg(h->device);
+    TLM_TRY(prepare(h));
+    *steps = 1;
+    if (pairAllowed(h))
+    {
+        TLM_TRY(ensurePair(h));
+        if (h->pair) *steps = 2;
+    }
+    return TLM_OK;
+}
+
 tlm_status tlm_kernel_time(tlm_handle h, double *ms, long long *launches)
 {
     TLM_TRY(checkHandle(h));
@@ -2217,7 +2462,7 @@ tlm_status tlm_kernel_time(tlm_handle h, double *ms, long long *launches)
         tot += m;
     }
     if (ms) *ms = tot;
-    if (launches) *launches = (long long)(h->evUsed / 2);
+    if (launches) *launches = h->timedSteps;
     return TLM_OK;
 }
 

@@ -550,6 +550,12 @@ class TlmSolver:
         self._c(self._L.tlm_step_launches(self._h, C.byref(n)))
         return n.value
 
+    def stepsPerPass(self) -> int:
+        """Steps per pass over the state (2 on large FP32 grids, else 1)."""
+        n = C.c_int(0)
+        self._c(self._L.tlm_steps_per_pass(self._h, C.byref(n)))
+        return n.value
+
     def kernelTime(self):
         ms = C.c_double(0)
         n = C.c_longlong(0)

@@ -453,7 +453,7 @@ def run_fdtd(args):
     ms = e0.elapsed_time(e1)
     s.close()
     n = w.ncells
-    bytes_step = n * (75 + 24)   # H: E read + H read/write; E: H read + E read/write + masks + lossy coefficients
+    bytes_step = n * 52   # one pass: E and H read and written, one word of edge classes
     achieved = bytes_step / (ms / args.steps / 1000.0) / 1e9
     peak, kind = peaks()
     t0 = time.perf_counter()

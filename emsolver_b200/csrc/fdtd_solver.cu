@@ -13,22 +13,30 @@
 //      coefficients), then the first-order Mur boundary in two launches whose
 //      order reproduces the reference's six face passes (edges shared by two
 //      faces end with the later pass's value).
-// Fields use the reference's Yee layouts (x fastest), so every update is a
-// coalesced row sweep; all arithmetic is FP32 in the reference's operation
-// order (the library is compiled with --fmad=false), hence bitwise results.
+// Steps 3 and 4 are one pass over memory (fusedStepKernel) from one field
+// buffer to another, and a Mur kernel that takes the old boundary values from
+// the input buffer; without room for a second field buffer they run in place,
+// one sweep for H and one for E.
+// Fields: one plane set per component, all six with the same pitch (cell
+// (i, j, k) of every component at (k*(ny+1) + j)*px + i; entries that a
+// component does not have stay zero). All arithmetic is FP32 in the
+// reference's operation order (the library is compiled with --fmad=false),
+// hence bitwise results.
 #include "fdtd_b200.h"
 #include "tlm_b200.h"
 #include "tlm_internal.h"
 
 #include "tlm_host_math.h"
-#include "tlm_device.cuh"
+#include "tlm_step_kernel.cuh"
 
 #include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <string>
+#include <tuple>
 #include <vector>
 
 using tlmi::SurfaceState;
@@ -38,30 +46,38 @@ namespace fdk {
 struct Dims
 {
     int nx, ny, nz;
-    __host__ __device__ long long iEx(int i, int j, int k) const { return ((long long)k * (ny + 1) + j) * nx + i; }
-    __host__ __device__ long long iEy(int i, int j, int k) const { return ((long long)k * ny + j) * (nx + 1) + i; }
-    __host__ __device__ long long iEz(int i, int j, int k) const
+    int px;  // row pitch: nx + 1 rounded up to 4
+    __host__ __device__ long long at(int i, int j, int k) const { return ((long long)k * (ny + 1) + j) * px + i; }
+    __host__ __device__ long long iEx(int i, int j, int k) const { return at(i, j, k); }
+    __host__ __device__ long long iEy(int i, int j, int k) const { return at(i, j, k); }
+    __host__ __device__ long long iEz(int i, int j, int k) const { return at(i, j, k); }
+    __host__ __device__ long long iHx(int i, int j, int k) const { return at(i, j, k); }
+    __host__ __device__ long long iHy(int i, int j, int k) const { return at(i, j, k); }
+    __host__ __device__ long long iHz(int i, int j, int k) const { return at(i, j, k); }
+    // 32-bit form for the in-place sweeps: setup refuses grids whose
+    // (nx+1)(ny+1)(nz+1) index box reaches 2^31, and the pitch adds at most a third.
+    __device__ unsigned q(int i, int j, int k) const
     {
-        return ((long long)k * (ny + 1) + j) * (nx + 1) + i;
+        return ((unsigned)k * (unsigned)(ny + 1) + (unsigned)j) * (unsigned)px + (unsigned)i;
     }
-    __host__ __device__ long long iHx(int i, int j, int k) const { return ((long long)k * ny + j) * (nx + 1) + i; }
-    __host__ __device__ long long iHy(int i, int j, int k) const { return ((long long)k * (ny + 1) + j) * nx + i; }
-    __host__ __device__ long long iHz(int i, int j, int k) const { return ((long long)k * ny + j) * nx + i; }
-    // 32-bit forms for the update sweeps: setup refuses grids whose
-    // (nx+1)(ny+1)(nz+1) index box reaches 2^31, so every component fits.
-    __device__ int jEx(int i, int j, int k) const { return (k * (ny + 1) + j) * nx + i; }
-    __device__ int jEy(int i, int j, int k) const { return (k * ny + j) * (nx + 1) + i; }
-    __device__ int jEz(int i, int j, int k) const { return (k * (ny + 1) + j) * (nx + 1) + i; }
-    __device__ int jHx(int i, int j, int k) const { return (k * ny + j) * (nx + 1) + i; }
-    __device__ int jHy(int i, int j, int k) const { return (k * (ny + 1) + j) * nx + i; }
-    __device__ int jHz(int i, int j, int k) const { return (k * ny + j) * nx + i; }
 };
+
+// Class of an E edge, ten bits per component (x, y, z from the low bits up) in
+// a word per cell: kEdgePec, kEdgeAir (the four cells around it are air), the
+// id of the dielectric that fills all four, from kEdgeFirst on a pair of
+// coefficients that edges between materials have, or, where the table has no
+// room for more of those, kEdgeMixed: coefficients in ca / cb. The table holds
+// the coefficients of every class below kEdgeMixed.
+enum : unsigned { kEdgePec = 0, kEdgeAir = 1, kEdgeFirst = 256, kEdgeMixed = 511, kEdgeClasses = 512 };
+__host__ __device__ __forceinline__ constexpr unsigned edgeWord(unsigned c) { return c * 0x00100401u; }  // all three
+__device__ __forceinline__ unsigned edgeClass(unsigned word, int comp) { return (word >> (10 * comp)) & 1023u; }
 
 struct Fields
 {
     float *E[3], *H[3];
-    const uint8_t *mE[3];        // 1 = free edge, 0 = PEC
-    const float *ca[3], *cb[3];  // lossy coefficients (nullptr: air everywhere)
+    const unsigned *cls;         // edge classes
+    const float2 *tab;           // (ca, cb) of every class but kEdgeMixed
+    const float *ca[3], *cb[3];  // of mixed edges (nullptr: no dielectric)
 };
 
 // ---- cell-centred averages (FdtdSolver.cpp:42-79) -------------------------
@@ -86,19 +102,28 @@ __device__ __forceinline__ float hcAt(const Fields &f, const Dims &d, int i, int
 // ---- 1. soft sources ----------------------------------------------------
 // Edge e (code: component * 2^60 + field index) receives amps[off[e]..off[e+1])
 // in source order: E += (-0.25 amp) sv each (FdtdSolver.cpp:404-437).
-__global__ void injectKernel(Fields f, const long long *__restrict__ edge, const int *__restrict__ off,
-                             const float *__restrict__ amps, int nedges, float sv)
+struct InjectArgs
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nedges) return;
-    const long long code = edge[e];
+    float *E[3];
+    const long long *edge;
+    const int *off;
+    const float *amps;
+    int nedges;
+    float sv;
+};
+__device__ __forceinline__ void injectItem(const InjectArgs &a, int e)
+{
+    if (e >= a.nedges) return;
+    const long long code = a.edge[e];
     const int c = (int)(code >> 60);
     const long long idx = code & ((1LL << 60) - 1);
-    float *E = c == 0 ? f.E[0] : c == 1 ? f.E[1] : f.E[2];
+    const int t0 = a.off[e], t1 = a.off[e + 1];
+    float *E = c == 0 ? a.E[0] : c == 1 ? a.E[1] : a.E[2];
     float v = E[idx];
-    for (int t = off[e]; t < off[e + 1]; ++t) v = v + (-0.25f * amps[t]) * sv;
+    for (int t = t0; t < t1; ++t) v = v + (-0.25f * a.amps[t]) * a.sv;
     E[idx] = v;
 }
+__global__ void injectKernel(const InjectArgs a) { injectItem(a, blockIdx.x * blockDim.x + threadIdx.x); }
 
 // ---- 2. monitors ----------------------------------------------------------
 struct MonArgs
@@ -130,16 +155,17 @@ struct MonArgs
     float *plane;
 };
 
+// (cells number below 2^31: 32-bit divisions)
 __device__ __forceinline__ void cellCo(long long c, const Dims &d, int co[3])
 {
-    co[0] = (int)(c % d.nx);
-    co[1] = (int)((c / d.nx) % d.ny);
-    co[2] = (int)(c / ((long long)d.nx * d.ny));
+    const unsigned u = (unsigned)c, r = u / (unsigned)d.nx, k = r / (unsigned)d.ny;
+    co[0] = (int)(u - r * (unsigned)d.nx);
+    co[1] = (int)(r - k * (unsigned)d.ny);
+    co[2] = (int)k;
 }
 
-__global__ void __launch_bounds__(256) monitorKernel(const MonArgs a)
+__device__ __forceinline__ void monitorItem(const MonArgs &a, long long t)
 {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const Fields &f = a.f;
     const Dims &d = a.d;
     if (t < a.nports)
@@ -251,6 +277,11 @@ __global__ void __launch_bounds__(256) monitorKernel(const MonArgs a)
     }
 }
 
+__global__ void __launch_bounds__(256) monitorKernel(const MonArgs a)
+{
+    monitorItem(a, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 // Energy (FdtdSolver.cpp:836-870): sum E^2 + eta0^2 sum H^2 in FP64, block
 // partials in a fixed order. Every component is swept as 16-byte vectors
 // (device allocations are 256-byte aligned), four in flight per thread.
@@ -276,13 +307,11 @@ __device__ __forceinline__ double sumSquares(const float *arr, long long n)
     }
     return acc;
 }
-__global__ void __launch_bounds__(256) energyPartialKernel(Fields f, long long nE0, long long nE1, long long nE2,
-                                                           long long nH0, long long nH1, long long nH2,
-                                                           double eta2, double *part)
+__global__ void __launch_bounds__(256) energyPartialKernel(Fields f, long long P, double eta2, double *part)
 {
     __shared__ double red[8];
-    const double se = (sumSquares(f.E[0], nE0) + sumSquares(f.E[1], nE1)) + sumSquares(f.E[2], nE2);
-    const double sh = (sumSquares(f.H[0], nH0) + sumSquares(f.H[1], nH1)) + sumSquares(f.H[2], nH2);
+    const double se = (sumSquares(f.E[0], P) + sumSquares(f.E[1], P)) + sumSquares(f.E[2], P);
+    const double sh = (sumSquares(f.H[0], P) + sumSquares(f.H[1], P)) + sumSquares(f.H[2], P);
     double s = se + sh * eta2;
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -349,21 +378,21 @@ struct MurAt
     float *s;
 };
 template <int F0, int NP>
-__device__ __forceinline__ bool murItem(const Mur &m, long long t, MurAt *a)
+__device__ __forceinline__ bool murItem(const Mur &m, unsigned t, MurAt *a)
 {
     bool found = false;
 #pragma unroll
     for (int p = F0; p < F0 + NP; ++p)
     {
-        const long long n = (long long)m.n1[p] * m.n2[p];
+        const unsigned n = (unsigned)m.n1[p] * (unsigned)m.n2[p];
         if (!found)
         {
             if (t < n)
             {
                 found = true;
                 a->F = p;
-                a->q1 = (int)(t % m.n1[p]);
-                a->q2 = (int)(t / m.n1[p]);
+                a->q2 = (int)(t / (unsigned)m.n1[p]);
+                a->q1 = (int)(t - (unsigned)a->q2 * (unsigned)m.n1[p]);
                 a->pl = n;
                 a->s = m.snap + m.off[p] + (long long)a->q2 * m.n1[p] + a->q1;
             }
@@ -376,7 +405,7 @@ __device__ __forceinline__ bool murItem(const Mur &m, long long t, MurAt *a)
 
 // Copy of layers 0, 1, N-1, N of every face plane, taken before the E
 // update (it runs as extra blocks of the H update, which leaves E unchanged).
-__device__ __forceinline__ void murSnapItem(const Fields &f, const Dims &d, const Mur &m, long long t)
+__device__ __forceinline__ void murSnapItem(const Fields &f, const Dims &d, const Mur &m, unsigned t)
 {
     MurAt a;
     if (!murItem<0, 6>(m, t, &a)) return;
@@ -418,7 +447,7 @@ __global__ void __launch_bounds__(256) updateHKernel(Fields f, Dims d, Box b, fl
 {
     if (blockIdx.x >= hBlocks)
     {
-        murSnapItem(f, d, m, (long long)(blockIdx.x - hBlocks) * blockDim.x + threadIdx.x);
+        murSnapItem(f, d, m, (blockIdx.x - hBlocks) * blockDim.x + threadIdx.x);
         return;
     }
     int i, j, k;
@@ -429,37 +458,44 @@ __global__ void __launch_bounds__(256) updateHKernel(Fields f, Dims d, Box b, fl
     const bool ax = j < d.ny && k < d.nz, ay = i < d.nx && k < d.nz, az = i < d.nx && j < d.ny;
     float hx = 0.f, hy = 0.f, hz = 0.f;
     float ez0 = 0.f, ezj = 0.f, ezi = 0.f, ey0 = 0.f, eyk = 0.f, eyi = 0.f, ex0 = 0.f, exk = 0.f, exj = 0.f;
-    const int qx = ax ? d.jHx(i, j, k) : 0, qy = ay ? d.jHy(i, j, k) : 0, qz = az ? d.jHz(i, j, k) : 0;
+    const unsigned q = d.q(i, j, k), qj = q + (unsigned)d.px, qk = q + (unsigned)d.px * (unsigned)(d.ny + 1);
     if (ax)
     {
-        hx = f.H[0][qx];
-        ezj = Ez[d.jEz(i, j + 1, k)];
-        eyk = Ey[d.jEy(i, j, k + 1)];
+        hx = f.H[0][q];
+        ezj = Ez[qj];
+        eyk = Ey[qk];
     }
     if (ay)
     {
-        hy = f.H[1][qy];
-        exk = Ex[d.jEx(i, j, k + 1)];
-        ezi = Ez[d.jEz(i + 1, j, k)];
+        hy = f.H[1][q];
+        exk = Ex[qk];
+        ezi = Ez[q + 1];
     }
     if (az)
     {
-        hz = f.H[2][qz];
-        eyi = Ey[d.jEy(i + 1, j, k)];
-        exj = Ex[d.jEx(i, j + 1, k)];
+        hz = f.H[2][q];
+        eyi = Ey[q + 1];
+        exj = Ex[qj];
     }
-    if (ax || ay) ez0 = Ez[d.jEz(i, j, k)];
-    if (ax || az) ey0 = Ey[d.jEy(i, j, k)];
-    if (ay || az) ex0 = Ex[d.jEx(i, j, k)];
-    if (ax) f.H[0][qx] = hx - ch * ((ezj - ez0) - (eyk - ey0));
-    if (ay) f.H[1][qy] = hy - ch * ((exk - ex0) - (ezi - ez0));
-    if (az) f.H[2][qz] = hz - ch * ((eyi - ey0) - (exj - ex0));
+    if (ax || ay) ez0 = Ez[q];
+    if (ax || az) ey0 = Ey[q];
+    if (ay || az) ex0 = Ex[q];
+    if (ax) f.H[0][q] = hx - ch * ((ezj - ez0) - (eyk - ey0));
+    if (ay) f.H[1][q] = hy - ch * ((exk - ex0) - (ezi - ez0));
+    if (az) f.H[2][q] = hz - ch * ((eyi - ey0) - (exj - ex0));
 }
 
-// E update of the interior edges (FdtdSolver.cpp:487-555). As for H, all
-// loads (masks, 6 distinct H values shared by the three components, the
-// edges' own E and lossy coefficients) come before the stores.
-__global__ void __launch_bounds__(256) updateEKernel(Fields f, Dims d, Box b, float cb0)
+// The coefficients of an edge of class c at index q.
+__device__ __forceinline__ float2 edgeCoef(const Fields &f, const float2 *tab, int comp, unsigned c, long long q)
+{
+    return c == kEdgeMixed ? make_float2(f.ca[comp][q], f.cb[comp][q]) : tab[c];
+}
+
+// E update of the interior edges (FdtdSolver.cpp:487-555), in place. As for
+// H, the loads (classes, 6 distinct H values shared by the three components,
+// the edges' own E) come before the stores. The update ca*E + cb*curl with the
+// air class's ca = 1 is the reference's E + cb0*curl.
+__global__ void __launch_bounds__(256) updateEKernel(Fields f, Dims d, Box b)
 {
     int i, j, k;
     if (!boxCell(b, d, &i, &j, &k)) return;
@@ -468,64 +504,50 @@ __global__ void __launch_bounds__(256) updateEKernel(Fields f, Dims d, Box b, fl
     const float *__restrict__ Hz = f.H[2];
     const bool ix = i >= 1 && i < d.nx, jy = j >= 1 && j < d.ny, kz = k >= 1 && k < d.nz;
     const bool ax = i < d.nx && jy && kz, ay = ix && j < d.ny && kz, az = ix && jy && k < d.nz;
-    const bool lossy = f.ca[0] != nullptr;
-    const int qx = ax ? d.jEx(i, j, k) : 0, qy = ay ? d.jEy(i, j, k) : 0, qz = az ? d.jEz(i, j, k) : 0;
-    uint8_t mx = 0, my = 0, mz = 0;
-    float ex = 0.f, ey = 0.f, ez = 0.f, cax = 0.f, cbx = 0.f, cay = 0.f, cby = 0.f, caz = 0.f, cbz = 0.f;
-    float hz0 = 0.f, hzj = 0.f, hzi = 0.f, hy0 = 0.f, hyk = 0.f, hyi = 0.f, hx0 = 0.f, hxk = 0.f, hxj = 0.f;
+    if (!ax && !ay && !az) return;
+    const unsigned q = d.q(i, j, k), qj = q - (unsigned)d.px, qk = q - (unsigned)d.px * (unsigned)(d.ny + 1);
+    const unsigned c = f.cls[q];
+    float ex = 0.f, ey = 0.f, ez = 0.f;
+    float hzj = 0.f, hzi = 0.f, hyk = 0.f, hyi = 0.f, hxk = 0.f, hxj = 0.f;
     if (ax)
     {
-        mx = f.mE[0][qx];
-        ex = f.E[0][qx];
-        hzj = Hz[d.jHz(i, j - 1, k)];
-        hyk = Hy[d.jHy(i, j, k - 1)];
-        if (lossy)
-        {
-            cax = f.ca[0][qx];
-            cbx = f.cb[0][qx];
-        }
+        ex = f.E[0][q];
+        hzj = Hz[qj];
+        hyk = Hy[qk];
     }
     if (ay)
     {
-        my = f.mE[1][qy];
-        ey = f.E[1][qy];
-        hxk = Hx[d.jHx(i, j, k - 1)];
-        hzi = Hz[d.jHz(i - 1, j, k)];
-        if (lossy)
-        {
-            cay = f.ca[1][qy];
-            cby = f.cb[1][qy];
-        }
+        ey = f.E[1][q];
+        hxk = Hx[qk];
+        hzi = Hz[q - 1];
     }
     if (az)
     {
-        mz = f.mE[2][qz];
-        ez = f.E[2][qz];
-        hyi = Hy[d.jHy(i - 1, j, k)];
-        hxj = Hx[d.jHx(i, j - 1, k)];
-        if (lossy)
-        {
-            caz = f.ca[2][qz];
-            cbz = f.cb[2][qz];
-        }
+        ez = f.E[2][q];
+        hyi = Hy[q - 1];
+        hxj = Hx[qj];
     }
-    if (ax || ay) hz0 = Hz[d.jHz(i, j, k)];
-    if (ax || az) hy0 = Hy[d.jHy(i, j, k)];
-    if (ay || az) hx0 = Hx[d.jHx(i, j, k)];
+    const float hx0 = Hx[q], hy0 = Hy[q], hz0 = Hz[q];
     if (ax)
     {
+        const unsigned cl = edgeClass(c, 0);
+        const float2 co = edgeCoef(f, f.tab, 0, cl, q);
         const float curl = (hz0 - hzj) - (hy0 - hyk);
-        f.E[0][qx] = !mx ? 0.0f : lossy ? cax * ex + cbx * curl : ex + cb0 * curl;
+        f.E[0][q] = cl == kEdgePec ? 0.0f : co.x * ex + co.y * curl;
     }
     if (ay)
     {
+        const unsigned cl = edgeClass(c, 1);
+        const float2 co = edgeCoef(f, f.tab, 1, cl, q);
         const float curl = (hx0 - hxk) - (hz0 - hzi);
-        f.E[1][qy] = !my ? 0.0f : lossy ? cay * ey + cby * curl : ey + cb0 * curl;
+        f.E[1][q] = cl == kEdgePec ? 0.0f : co.x * ey + co.y * curl;
     }
     if (az)
     {
+        const unsigned cl = edgeClass(c, 2);
+        const float2 co = edgeCoef(f, f.tab, 2, cl, q);
         const float curl = (hy0 - hyi) - (hx0 - hxj);
-        f.E[2][qz] = !mz ? 0.0f : lossy ? caz * ez + cbz * curl : ez + cb0 * curl;
+        f.E[2][q] = cl == kEdgePec ? 0.0f : co.x * ez + co.y * curl;
     }
 }
 
@@ -535,7 +557,7 @@ template <int F0>
 __global__ void murApplyKernel(Fields f, Dims d, Mur m)
 {
     MurAt a;
-    if (!murItem<F0, 3>(m, (long long)blockIdx.x * blockDim.x + threadIdx.x, &a)) return;
+    if (!murItem<F0, 3>(m, blockIdx.x * blockDim.x + threadIdx.x, &a)) return;
     const int N = murN(d, a.F);
     float *E = murField(f, a.F);
     const long long b0 = murIndex(d, a.F, 0, a.q1, a.q2), b1 = murIndex(d, a.F, 1, a.q1, a.q2);
@@ -546,9 +568,446 @@ __global__ void murApplyKernel(Fields f, Dims d, Mur m)
     E[bN] = s2 + m.cMur * (eN1 - s3);
 }
 
+// ---- 3 and 4 in one pass ---------------------------------------------------
+// A block owns a column of TX x TY cells and walks a range of z planes. On
+// every plane it computes the new H of the column and of the ring below it in
+// x and y (the ring is computed by the neighbouring blocks as well), hands it
+// to the block through shared memory (two buffers, one barrier per plane), and
+// computes the new E from it and from the H of the plane below, which each
+// thread keeps in registers. A thread owns two x-neighbours (packed FP32x2
+// arithmetic, bitwise the scalar operations).
+// The input planes come in by tensor-map bulk copies, three boxes per plane:
+// Ex and Ey one plane ahead, Ez, and H. A stage's Ex and Ey serve two planes
+// (as the plane above, then as the plane itself), so a stage is refilled two
+// planes after its own; with three stages the next plane is always in flight.
+// Per cell and step this reads E, H and one class word and writes E and H: 52
+// bytes, against 99 for two sweeps with per-edge coefficients. Planes whose
+// edges are all air (a flag per column and plane) read no classes.
+template <int W_, int H_> struct FusedLayout
+{
+    static constexpr int W = W_, H = H_;  // pairs x rows of threads: the column and its ring
+    static constexpr int maxTX = 2 * (W - 1) / 4 * 4, maxTY = H - 1;
+    static constexpr int kThreads = (W * H + 31) / 32 * 32, kStages = 3;
+    // a stage row holds the W2 cells from x0-4 on (16-byte aligned box starts); floats
+    static constexpr int W2 = (2 * W + 4 + 3) / 4 * 4;
+    static constexpr int round32(int f) { return (f + 31) / 32 * 32; }  // boxes start on 128-byte boundaries
+    static constexpr int sE = (H + 1) * W2, sH = H * W2;
+    static constexpr int offEz = round32(2 * sE), offH = offEz + round32(sE), stage = offH + round32(3 * sH);
+    static constexpr unsigned stageBytes = (unsigned)(3 * sE + 3 * sH) * 4u;
+    static constexpr int WE = 2 * W, slot = H * WE;  // exchange row and slot
+    static constexpr int offEx = kStages * stage, offTab = offEx + 2 * 3 * slot;
+    static constexpr int smemBytes = (offTab + 2 * kEdgeClasses) * 4;
+    static constexpr int kFit = 227 * 1024 / (smemBytes + 1280);
+    static constexpr int kMinBlocks = 1024 / kThreads < kFit ? 1024 / kThreads : kFit;
+    static_assert(kMinBlocks >= 1, "a block fits an SM");
+};
+struct FusedArgs
+{
+    CUtensorMap mapExy, mapEz, mapH;  // boxes of the input buffer
+    Fields in;
+    float *out;       // Ex Ey Ez Hx Hy Hz planes of P values each
+    long long P;
+    Dims d;
+    int TX, TY, ntx, nty, nchunk;
+    const unsigned char *flags;  // [column][nz + 1]: some edge is not air
+    float ch, cb0, neg_zero;
+    unsigned *fault;
+};
+
+using tlmk::add2;
+using tlmk::ld2;
+using tlmk::mul2;
+using tlmk::splat2;
+using tlmk::sub2;
+
+template <class L> __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) fusedStepKernel(const __grid_constant__ FusedArgs a)
+{
+    extern __shared__ __align__(128) float sm[];
+    __shared__ __align__(8) unsigned long long full[L::kStages];
+    const Dims &d = a.d;
+    const int tid = threadIdx.x;
+    const int ncol = a.ntx * a.nty;
+    const int col = blockIdx.x % ncol, chunk = blockIdx.x / ncol;
+    const int planes = d.nz + 1;
+    const int kc0 = (int)((long long)chunk * planes / a.nchunk), kc1 = (int)((long long)(chunk + 1) * planes / a.nchunk);
+    const int kA = kc0 > 0 ? kc0 - 1 : 0;
+    const int x0 = (col % a.ntx) * a.TX, y0 = (col / a.ntx) * a.TY;
+    const unsigned full0 = tlmk::smemAddr(full), sm0 = tlmk::smemAddr(sm);
+    if (tid == 0)
+    {
+        for (int s = 0; s < L::kStages; ++s)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" : : "r"(full0 + 8 * s) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" : : : "memory");
+    }
+    float2 *const tab = reinterpret_cast<float2 *>(sm + L::offTab);
+    for (int t = tid; t < (int)kEdgeClasses; t += L::kThreads) tab[t] = a.in.tab[t];
+    __syncthreads();
+    // stage of plane k (k from kA-1: only its Ex and Ey, those of plane kA, are used)
+    auto issue = [&](int k) {
+        const int s = (k - kA + 1) % L::kStages;
+        const unsigned st = sm0 + (unsigned)(s * L::stage) * 4u, bar = full0 + 8 * s;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" : : "r"(bar), "r"(L::stageBytes) : "memory");
+        tlmk::tmaBox4(st, &a.mapExy, x0 - 4, y0 - 1, k + 1, 0, bar);
+        tlmk::tmaBox4(st + L::offEz * 4u, &a.mapEz, x0 - 4, y0 - 1, k, 2, bar);
+        tlmk::tmaBox4(st + L::offH * 4u, &a.mapH, x0 - 4, y0 - 1, k, 3, bar);
+    };
+    int lastIssued = kA - 2;  // thread 0's
+    if (tid == 0)
+        while (lastIssued < kc1 - 1 && lastIssued < kA - 2 + L::kStages) issue(++lastIssued);
+
+    const int r = tid / L::W, p = tid - r * L::W;
+    const bool inTile = r < L::H;
+    const int i = x0 - 2 + 2 * p, j = y0 - 1 + r;
+    const bool own = inTile && p >= 1 && p <= a.TX / 2 && r >= 1 && r <= a.TY && i <= d.nx && j <= d.ny;
+    const unsigned off = own ? (unsigned)j * (unsigned)d.px + (unsigned)i : 0u;
+    const long long sz = (long long)d.px * (d.ny + 1);
+    const unsigned char *flags = a.flags + (long long)col * planes;
+    const bool i0 = i < d.nx, i1 = i + 1 < d.nx, up = j < d.ny;
+    const bool jy = j >= 1 && up;
+    // which of the pair's edges the E update writes (z conditions apart): bit
+    // 2*component + node
+    const bool iy = i >= 1 && up;
+    const unsigned eMask = (i0 && jy ? 1u : 0u) | (i1 && jy ? 2u : 0u) | (iy && i0 ? 4u : 0u) | (up && i1 ? 8u : 0u) |
+                           (i >= 1 && i0 && jy ? 16u : 0u) | (i1 && jy ? 32u : 0u);
+    const float2 z = splat2(a.neg_zero), ch = splat2(a.ch);
+    const int o = inTile ? r * L::W2 + 2 * p + 2 : 2;       // in a stage
+    const int e0 = L::offEx + (inTile ? r * L::WE + 2 * p : 0);  // in an exchange buffer
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 hxP = zero, hyP = zero;  // new H of the plane below
+    bool waitOk = true;
+    int sPrev = 0, sCur = 0;
+    unsigned phase = 0;
+    auto wait = [&]() {  // for the stage sCur
+        if (waitOk && !tlmk::mbarWaitBounded(full0 + 8 * sCur, phase))
+        {
+            waitOk = false;
+            atomicOr(a.fault, tlmk::kStageTimeout);
+        }
+    };
+    wait();
+    sCur = 1;
+    uint2 cNext = make_uint2(0, 0);
+    // classes one plane ahead, the flags that say whether there are any three
+    auto flagAt = [&](int k) -> unsigned { return k < kc1 ? flags[k] : 0u; };
+    auto classesAt = [&](int k, unsigned f) -> uint2 {
+        return f && own ? *reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(a.in.cls + k * sz) + off * 4u)
+                        : make_uint2(0, 0);
+    };
+    unsigned f0 = flagAt(kA), f1 = flagAt(kA + 1), f2 = flagAt(kA + 2);
+    cNext = classesAt(kA, f0);
+    // lanes with cells at the high x and y faces, where some entries do not exist
+    const bool warpHigh = __any_sync(0xffffffffu, !i1 || !up);
+    for (int k = kA; k < kc1; ++k)
+    {
+        const bool kz = k < d.nz;
+        const unsigned f3 = flagAt(k + 3);
+        const uint2 c = cNext;
+        cNext = classesAt(k + 1, f1);
+        wait();
+        const float *prev = sm + sPrev * L::stage, *st = sm + sCur * L::stage;
+        // ---- H (FdtdSolver.cpp:449-484) ----
+        const float2 ex = ld2(prev + o), ey = ld2(prev + L::sE + o), ez = ld2(st + L::offEz + o);
+        const float2 exj = ld2(prev + o + L::W2), ezj = ld2(st + L::offEz + o + L::W2);
+        const float2 ey1 = make_float2(prev[L::sE + o + 1], prev[L::sE + o + 2]);
+        const float2 ez1 = make_float2(st[L::offEz + o + 1], st[L::offEz + o + 2]);
+        const float2 exk = ld2(st + o), eyk = ld2(st + L::sE + o);
+        float2 hx = ld2(st + L::offH + o), hy = ld2(st + L::offH + L::sH + o), hz = ld2(st + L::offH + 2 * L::sH + o);
+        hx = sub2(hx, mul2(ch, sub2(sub2(ezj, ez), sub2(eyk, ey)), z));
+        hy = sub2(hy, mul2(ch, sub2(sub2(exk, ex), sub2(ez1, ez)), z));
+        hz = sub2(hz, mul2(ch, sub2(sub2(ey1, ey), sub2(exj, ex)), z));
+        // entries a component does not have stay zero
+        if (warpHigh || !kz)
+        {
+            if (!up || !kz) hx = zero;
+            if (!up) hz = zero;
+            if (!kz) hy = zero;
+            if (!i0) hy.x = hz.x = 0.f;
+            if (!i1) hy.y = hz.y = 0.f;
+            if (i >= d.nx) hx.y = 0.f;
+        }
+        float *const xb = sm + (k & 1) * 3 * L::slot + e0;
+        if (inTile)
+        {
+            *reinterpret_cast<float2 *>(xb) = hx;
+            *reinterpret_cast<float2 *>(xb + L::slot) = hy;
+            *reinterpret_cast<float2 *>(xb + 2 * L::slot) = hz;
+        }
+        __syncthreads();
+        // every thread is past its reads of the stage before this one's
+        if (tid == 0 && waitOk && lastIssued < kc1 - 1 && lastIssued < k + L::kStages - 1) issue(++lastIssued);
+        if (own && k >= kc0)
+        {
+            // uniform plane pointers and a 32-bit lane offset
+            char *const out = reinterpret_cast<char *>(a.out + k * sz);
+            auto store = [&](int comp, float2 v) { *reinterpret_cast<float2 *>(out + comp * a.P * 4 + off * 4u) = v; };
+            store(3, hx);
+            store(4, hy);
+            store(5, hz);
+            // ---- E of the interior edges (FdtdSolver.cpp:487-555) ----
+            const float2 hxj = ld2(xb - L::WE), hzj = ld2(xb + 2 * L::slot - L::WE);
+            const float2 hyi = make_float2(xb[L::slot - 1], xb[L::slot]);
+            const float2 hzi = make_float2(xb[2 * L::slot - 1], xb[2 * L::slot]);
+            const float2 cx = sub2(sub2(hz, hzj), sub2(hy, hyP));
+            const float2 cy = sub2(sub2(hx, hxP), sub2(hz, hzi));
+            const float2 cz = sub2(sub2(hy, hyi), sub2(hx, hxj));
+            float2 nx, ny, nz;
+            const unsigned l = edgeClass(c.x, 0);
+            if (!f0)
+            {
+                const float2 cb = splat2(a.cb0);
+                nx = add2(ex, mul2(cb, cx, z));
+                ny = add2(ey, mul2(cb, cy, z));
+                nz = add2(ez, mul2(cb, cz, z));
+            }
+            else if (c.x == c.y && c.x == edgeWord(l) && l - 1u < kEdgeMixed - 1u)
+            {
+                // all six edges inside one material
+                const float2 co = tab[l], ca = splat2(co.x), cb = splat2(co.y);
+                nx = add2(mul2(ca, ex, z), mul2(cb, cx, z));
+                ny = add2(mul2(ca, ey, z), mul2(cb, cy, z));
+                nz = add2(mul2(ca, ez, z), mul2(cb, cz, z));
+            }
+            else
+            {
+                auto update = [&](int comp, float2 e, float2 curl) -> float2 {
+                    const unsigned l0 = edgeClass(c.x, comp), l1 = edgeClass(c.y, comp);
+                    const long long q = k * sz + off;
+                    const float2 k0 = edgeCoef(a.in, tab, comp, l0, q), k1 = edgeCoef(a.in, tab, comp, l1, q + 1);
+                    float2 v = add2(mul2(make_float2(k0.x, k1.x), e, z), mul2(make_float2(k0.y, k1.y), curl, z));
+                    if (l0 == kEdgePec) v.x = 0.f;
+                    if (l1 == kEdgePec) v.y = 0.f;
+                    return v;
+                };
+                nx = update(0, ex, cx);
+                ny = update(1, ey, cy);
+                nz = update(2, ez, cz);
+            }
+            // boundary edges are written by the Mur kernel
+            const bool kin = k >= 1 && kz;
+            if (eMask == 63u && kin)
+            {
+                store(0, nx);
+                store(1, ny);
+                store(2, nz);
+            }
+            else
+            {
+                auto masked = [&](int comp, float2 v) {
+                    const unsigned m = (eMask >> (2 * comp)) & 3u;
+                    if (m) store(comp, make_float2((m & 1u) ? v.x : 0.f, (m & 2u) ? v.y : 0.f));
+                };
+                if (kin)
+                {
+                    masked(0, nx);
+                    masked(1, ny);
+                }
+                if (kz) masked(2, nz);
+            }
+        }
+        f0 = f1;
+        f1 = f2;
+        f2 = f3;
+        hxP = hx;
+        hyP = hy;
+        sPrev = sCur;
+        if (++sCur == L::kStages)
+        {
+            sCur = 0;
+            phase ^= 1u;
+        }
+    }
+    // Thread 0 waited for every copy, unless a wait ran out: then let those
+    // still in flight land before the block's memory goes.
+    if (!waitOk && tid == 0)
+        for (int k = max(kA - 1, lastIssued - L::kStages + 1); k <= lastIssued; ++k)
+            tlmk::mbarWaitBounded(full0 + 8 * ((k - kA + 1) % L::kStages),
+                                  (unsigned)((k - kA + 1) / L::kStages) & 1u);
+}
+
+// Mur on all faces at once, from the old values `o` (input buffer) and the
+// fused pass's new interior edges `n` (FdtdSolver.cpp:624-670). The reference
+// runs the face planes one after the other and a later one overwrites the edges
+// it shares with an earlier one, from an inner neighbour that the earlier one
+// may have set: an edge of two faces takes the later face's formula here, with
+// the earlier face's where the inner neighbour lies on that.
+__device__ __forceinline__ float murStep(const float *o, const float *n, long long b, long long inner, float c)
+{
+    return o[inner] + c * (n[inner] - o[b]);
+}
+__device__ __forceinline__ void murFaceItem(const float *oldE, float *newE, long long P, const Dims &d, const Mur &m,
+                                            unsigned t)
+{
+    MurAt a;
+    if (!murItem<0, 6>(m, t, &a)) return;
+    const int comp = (a.F == 0 || a.F == 5) ? 1 : (a.F == 1 || a.F == 3) ? 2 : 0;
+    const float *o = oldE + comp * P;
+    float *n = newE + comp * P;
+    // planes 0, 1, 2 leave the edges that a later plane of their component
+    // sets: (q1, q2) is (j, k) on planes 0, 1 and (i, k) on plane 2
+    if (a.F == 0 && (a.q2 == 0 || a.q2 == d.nz)) return;
+    if (a.F == 1 && (a.q1 == 0 || a.q1 == d.ny)) return;
+    if (a.F == 2 && (a.q2 == 0 || a.q2 == d.nz)) return;
+    const int N = murN(d, a.F);
+    for (int side = 0; side < 2; ++side)
+    {
+        const int b = side ? N : 0, q = side ? N - 1 : 1;
+        const long long ib = murIndex(d, a.F, b, a.q1, a.q2), iq = murIndex(d, a.F, q, a.q1, a.q2);
+        float v1;
+        if (a.F == 3 && (a.q1 == 0 || a.q1 == d.nx))  // inner edge on an x face (plane 1)
+            v1 = murStep(o, n, iq, d.iEz(a.q1 == 0 ? 1 : d.nx - 1, q, a.q2), m.cMur);
+        else if (a.F == 4 && (a.q2 == 0 || a.q2 == d.ny))  // on a y face (plane 2)
+            v1 = murStep(o, n, iq, d.iEx(a.q1, a.q2 == 0 ? 1 : d.ny - 1, q), m.cMur);
+        else if (a.F == 5 && (a.q1 == 0 || a.q1 == d.nx))  // on an x face (plane 0)
+            v1 = murStep(o, n, iq, d.iEy(a.q1 == 0 ? 1 : d.nx - 1, a.q2, q), m.cMur);
+        else
+            v1 = n[iq];
+        n[ib] = o[iq] + m.cMur * (v1 - o[ib]);
+    }
+}
+
+// What follows the fused pass of a step, in one launch: Mur on the new fields,
+// the step's monitors, which read the old ones, and, where none of the source
+// edges lies on an outer face or next to one (so that Mur does not read them),
+// the next step's sources.
+struct TailArgs
+{
+    const float *oldE;
+    float *newE;
+    long long P;
+    Mur mur;
+    MonArgs mon;
+    InjectArgs inj;
+    unsigned murBlocks, monBlocks;
+};
+__global__ void __launch_bounds__(256) stepTailKernel(const __grid_constant__ TailArgs a)
+{
+    if (blockIdx.x < a.murBlocks)
+        murFaceItem(a.oldE, a.newE, a.P, a.mon.d, a.mur, blockIdx.x * blockDim.x + threadIdx.x);
+    else if (blockIdx.x < a.murBlocks + a.monBlocks)
+        monitorItem(a.mon, (long long)(blockIdx.x - a.murBlocks) * blockDim.x + threadIdx.x);
+    else
+        injectItem(a.inj, (int)((blockIdx.x - a.murBlocks - a.monBlocks) * blockDim.x + threadIdx.x));
+}
+
+// ---- edge classes (FdtdSolver.cpp:135-231) ---------------------------------
+// A free table entry: (ca, cb) = (NaN, NaN), which no edge has.
+constexpr unsigned long long kEdgeFree = ~0ull;
+
+// One thread per cell of the index box: the classes of its three edges, and
+// the coefficients of those between materials, from the four cells around each (summed
+// in the reference's order). Edges on the outer boundary are not updated from
+// their classes.
+__global__ void __launch_bounds__(256) edgeClassKernel(const uint8_t *__restrict__ mat, const float2 *__restrict__ props,
+                                                       Dims d, Box b, float dt, float dl, float eps0, unsigned *cls,
+                                                       unsigned long long *tab,
+                                                       float *ca0, float *ca1, float *ca2, float *cb0, float *cb1,
+                                                       float *cb2)
+{
+    int i, j, k;
+    if (!boxCell(b, d, &i, &j, &k)) return;
+    unsigned word = 0;
+#pragma unroll
+    for (int axis = 0; axis < 3; ++axis)
+    {
+        unsigned c = kEdgeAir;
+        const int co[3] = { i, j, k };
+        const int n[3] = { d.nx, d.ny, d.nz };
+        const int t1 = axis == 0 ? 1 : 0, t2 = axis == 2 ? 1 : 2;
+        if (co[axis] < n[axis] && co[t1] >= 1 && co[t1] < n[t1] && co[t2] >= 1 && co[t2] < n[t2])
+        {
+            uint8_t m[4];
+            bool pec = false, same = true;
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+            {
+                int q[3] = { i, j, k };
+                q[t1] -= t < 2 ? 1 : 0;
+                q[t2] -= (t & 1) ? 0 : 1;
+                m[t] = mat[((size_t)q[2] * d.ny + q[1]) * d.nx + q[0]];
+                pec = pec || m[t] == TLM_MAT_PEC;
+                same = same && m[t] == m[0];
+            }
+            if (pec)
+                c = kEdgePec;
+            else if (same)
+                c = m[0] == TLM_MAT_AIR ? kEdgeAir : m[0];
+            else
+            {
+                float e = 0.0f, s = 0.0f;
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                {
+                    const float2 pr = m[t] >= TLM_MAT_DIEL0 ? props[m[t] - TLM_MAT_DIEL0] : make_float2(1.0f, 0.0f);
+                    e += m[t] >= TLM_MAT_DIEL0 ? 1.0f + (pr.x - 1.0f) : 1.0f;
+                    s += pr.y;
+                }
+                const float er = e / 4.0f, sg = s / 4.0f;
+                const float eps = eps0 * (1.0f < er ? er : 1.0f);
+                const float lf = sg * dt / (2.0f * eps);
+                const float ca = (1.0f - lf) / (1.0f + lf), cb = (dt / (eps * dl)) / (1.0f + lf);
+                // this pair's entry in the table, a new one if there is room
+                const unsigned long long key = (unsigned long long)__float_as_uint(cb) << 32 | __float_as_uint(ca);
+                c = kEdgeMixed;
+                constexpr unsigned kRoom = kEdgeMixed - kEdgeFirst;
+                const unsigned start = tlmk::mix32((unsigned)(key ^ (key >> 32))) % kRoom;
+                for (unsigned u = 0; u < kRoom; ++u)
+                {
+                    const unsigned t = kEdgeFirst + (start + u) % kRoom;
+                    unsigned long long old = reinterpret_cast<volatile unsigned long long *>(tab)[t];
+                    if (old == kEdgeFree) old = atomicCAS(tab + t, kEdgeFree, key);
+                    if (old == kEdgeFree || old == key)
+                    {
+                        c = t;
+                        break;
+                    }
+                }
+                if (c == kEdgeMixed)
+                {
+                    const long long q = d.at(i, j, k);
+                    (axis == 0 ? ca0 : axis == 1 ? ca1 : ca2)[q] = ca;
+                    (axis == 0 ? cb0 : axis == 1 ? cb1 : cb2)[q] = cb;
+                }
+            }
+        }
+        word |= c << (10 * axis);
+    }
+    cls[d.at(i, j, k)] = word;
+}
+// Columns and planes that hold an edge that is not air.
+__global__ void __launch_bounds__(128) edgeFlagKernel(const unsigned *__restrict__ cls, Dims d, int TX, int TY, int ntx,
+                                                      unsigned char *flags)
+{
+    const int k = blockIdx.x % (d.nz + 1), col = blockIdx.x / (d.nz + 1);
+    const int xa = (col % ntx) * TX, ya = (col / ntx) * TY;
+    const int w = min(TX, d.nx + 1 - xa), hgt = min(TY, d.ny + 1 - ya);
+    const unsigned air = edgeWord(kEdgeAir);
+    bool other = false;
+    for (int t = threadIdx.x; t < w * hgt; t += blockDim.x)
+        other = other || cls[d.at(xa + t % w, ya + t / w, k)] != air;
+    other = __syncthreads_or(other);
+    if (threadIdx.x == 0) flags[blockIdx.x] = other ? 1 : 0;
+}
+
+// A component of extents n in the reference's layout (x fastest, no padding).
+__global__ void __launch_bounds__(256) packFieldKernel(const float *__restrict__ f, Dims d, int n0, int n1, long long total,
+                                                       float *__restrict__ out)
+{
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+         t += (long long)gridDim.x * blockDim.x)
+    {
+        const int i = (int)(t % n0);
+        const long long r = t / n0;
+        out[t] = f[d.at(i, (int)(r % n1), (int)(r / n1))];
+    }
+}
+
 } // namespace fdk
 
 // ---------------------------------------------------------------------------
+struct FdtdMaps
+{
+    CUtensorMap map[2][3];  // per field buffer: Ex and Ey, Ez, H
+};
 struct fdtd_solver
 {
     int device = 0;
@@ -563,12 +1022,19 @@ struct fdtd_solver
     fdk::Dims d{};
     float dt = 0, cMur = 0, cb0 = 0, ch = 0;
     bool haveDiel = false;
-    long long len[6] = {};       // Ex Ey Ez Hx Hy Hz lengths
-    void *dField[6] = {};
-    uint8_t *dMask[3] = {};
-    std::vector<uint8_t> hMask[3];  // host copies of the PEC masks (source edges)
-    float *dCa[3] = {}, *dCb[3] = {};
+    long long len[6] = {};       // Ex Ey Ez Hx Hy Hz lengths in the reference's layout
+    long long P = 0;             // entries of a component's plane set (padded pitch)
+    float *dBuf[2] = {};         // field buffers of 6 P values; the second only for fused passes
+    int cur = 0;                 // buffer holding the current state
+    unsigned *dCls = nullptr;    // edge classes
+    float2 *dTab = nullptr;      // their coefficients
+    float *dCa[3] = {}, *dCb[3] = {};  // of mixed edges
+    unsigned char *dFlags = nullptr;   // [column][plane] of the fused pass
+    unsigned *dFault = nullptr;        // a bulk copy's wait ran out
+    std::unique_ptr<FdtdMaps> maps;    // boxes of the fused pass in either buffer
+    int layout = 0, TX = 0, TY = 0, ntx = 0, nty = 0, nchunk = 0;
     fdk::Mur mur{};
+    float *field(int c) const { return dBuf[cur] + c * P; }
     // sources
     struct Src
     {
@@ -591,6 +1057,8 @@ struct fdtd_solver
     int *dEdgeOff = nullptr;
     float *dAmps = nullptr;
     int nEdges = 0;
+    bool edgesInside = false;  // no source edge on an outer face or one cell from it
+    bool injected = false;     // the current state holds the next step's sources already
     int *dPoff = nullptr, *dPpol = nullptr;
     long long *dPcells = nullptr, *dProbe = nullptr;
     float *dVrec = nullptr, *dIrec = nullptr, *dPrec = nullptr;
@@ -601,7 +1069,23 @@ struct fdtd_solver
     int curStep = 0;
     std::vector<void *> allocs;
 
-    bool maskHost(int c, long long idx) const { return hMask[c][(size_t)idx] != 0; }
+    // whether the edge of component c at (i, j, k) touches no PEC cell
+    bool freeEdge(int c, int i, int j, int k) const
+    {
+        const int t1 = c == 0 ? 1 : 0, t2 = c == 2 ? 1 : 2;
+        const int n[3] = { d.nx, d.ny, d.nz };
+        for (int d1 = -1; d1 <= 0; ++d1)
+            for (int d2 = -1; d2 <= 0; ++d2)
+            {
+                int co[3] = { i, j, k };
+                co[t1] += d1;
+                co[t2] += d2;
+                bool in = true;
+                for (int a = 0; a < 3; ++a) in = in && co[a] >= 0 && co[a] < n[a];
+                if (in && mat[((size_t)co[2] * d.ny + co[1]) * d.nx + co[0]] == TLM_MAT_PEC) return false;
+            }
+        return true;
+    }
     tlm_status fail(tlm_status s, const std::string &m)
     {
         err = m;
@@ -694,10 +1178,14 @@ void freeMonitors(fdtd_solver *h)
 void freeAll(fdtd_solver *h)
 {
     freeMonitors(h);
-    for (int c = 0; c < 6; ++c) release(h, h->dField[c]);
+    for (int b = 0; b < 2; ++b) release(h, h->dBuf[b]);
+    release(h, h->dCls);
+    release(h, h->dTab);
+    release(h, h->dFlags);
+    release(h, h->dFault);
+    h->maps.reset();
     for (int c = 0; c < 3; ++c)
     {
-        release(h, h->dMask[c]);
         release(h, h->dCa[c]);
         release(h, h->dCb[c]);
     }
@@ -763,21 +1251,16 @@ tlm_status prepare(fdtd_solver *h)
     std::map<long long, std::vector<float>> edges;  // per edge, amplitudes in source order
     auto add = [&](uint64_t cell, int pol, float amp) {
         const int i = (int)(cell % d.nx), j = (int)((cell / d.nx) % d.ny), k = (int)(cell / ((uint64_t)d.nx * d.ny));
-        long long idx[4];
-        if (pol == 0)
-        {
-            idx[0] = d.iEx(i, j, k); idx[1] = d.iEx(i, j + 1, k); idx[2] = d.iEx(i, j, k + 1); idx[3] = d.iEx(i, j + 1, k + 1);
-        }
-        else if (pol == 1)
-        {
-            idx[0] = d.iEy(i, j, k); idx[1] = d.iEy(i + 1, j, k); idx[2] = d.iEy(i, j, k + 1); idx[3] = d.iEy(i + 1, j, k + 1);
-        }
-        else
-        {
-            idx[0] = d.iEz(i, j, k); idx[1] = d.iEz(i + 1, j, k); idx[2] = d.iEz(i, j + 1, k); idx[3] = d.iEz(i + 1, j + 1, k);
-        }
+        // the four edges along pol, by increasing second, then first transverse axis
+        const int t1 = pol == 0 ? 1 : 0, t2 = pol == 2 ? 1 : 2;
         for (int e = 0; e < 4; ++e)
-            if (h->maskHost(pol, idx[e])) edges[((long long)pol << 60) | idx[e]].push_back(amp);
+        {
+            int co[3] = { i, j, k };
+            co[t1] += e & 1;
+            co[t2] += e >> 1;
+            if (h->freeEdge(pol, co[0], co[1], co[2]))
+                edges[((long long)pol << 60) | d.at(co[0], co[1], co[2])].push_back(amp);
+        }
     };
     for (const auto &s : h->planeSources) add(s.cell, s.pol, s.amp);
     for (const auto &p : h->ports)
@@ -792,6 +1275,14 @@ tlm_status prepare(fdtd_solver *h)
         off.push_back((int)amps.size());
     }
     h->nEdges = (int)code.size();
+    h->edgesInside = true;
+    for (long long c : code)
+    {
+        const long long idx = c & ((1LL << 60) - 1);
+        const int co[3] = { (int)(idx % d.px), (int)(idx / d.px % (d.ny + 1)), (int)(idx / ((long long)d.px * (d.ny + 1))) };
+        const int n[3] = { d.nx, d.ny, d.nz };
+        for (int q = 0; q < 3; ++q) h->edgesInside = h->edgesInside && co[q] >= 2 && co[q] <= n[q] - 2;
+    }
     if (h->nEdges)
     {
         FD_TRY(alloc(h, &h->dEdge, code.size() * 8));
@@ -858,23 +1349,122 @@ tlm_status prepare(fdtd_solver *h)
     return TLM_OK;
 }
 
-tlm_status launchStep(fdtd_solver *h, int n)
+fdk::Box boxOf(const fdk::Dims &d)
+{
+    fdk::Box box;
+    box.total = (unsigned)((long long)(d.nx + 1) * (d.ny + 1) * (d.nz + 1));
+    box.divX = tlmk::makeFastDiv((unsigned)(d.nx + 1));
+    box.divY = tlmk::makeFastDiv((unsigned)(d.ny + 1));
+    return box;
+}
+
+using FusedLayouts = std::tuple<fdk::FusedLayout<51, 10>, fdk::FusedLayout<35, 14>, fdk::FusedLayout<17, 15>>;
+template <int I = 0, class F> void withFusedLayout(int layout, F &&f)
+{
+    if constexpr (I < (int)std::tuple_size<FusedLayouts>::value)
+    {
+        if (layout == I)
+            f(std::tuple_element_t<I, FusedLayouts>{});
+        else
+            withFusedLayout<I + 1>(layout, f);
+    }
+}
+
+// The columns of fused passes with the least cost: waves of resident blocks
+// times planes (one of them the ring's plane below) times a block's threads.
+void chooseFused(fdtd_solver *h, int sms)
+{
+    const fdk::Dims &d = h->d;
+    long long best = -1;
+    for (int l = 0; l < (int)std::tuple_size<FusedLayouts>::value; ++l)
+        withFusedLayout(l, [&](auto L) {
+            using Layout = decltype(L);
+            const int nx = d.nx + 1, ny = d.ny + 1, nz = d.nz + 1;
+            const int ntx = (nx + Layout::maxTX - 1) / Layout::maxTX;
+            const int TX = ((nx + ntx - 1) / ntx + 3) / 4 * 4;
+            const int rows0 = (ny + Layout::maxTY - 1) / Layout::maxTY;
+            for (int rows = rows0; rows < rows0 + 6 && rows <= ny; ++rows)
+            {
+                const int TY = (ny + rows - 1) / rows, nty = (ny + TY - 1) / TY;
+                for (int c = 1; c <= std::max(1, nz / 2); ++c)
+                {
+                    const long long slots = (long long)sms * Layout::kMinBlocks;
+                    const long long waves = ((long long)ntx * nty * c + slots - 1) / slots;
+                    const long long cost = waves * ((nz + c - 1) / c + (c > 1 ? 1 : 0)) *
+                                           (Layout::kThreads * Layout::kMinBlocks);
+                    if (best >= 0 && cost >= best) continue;
+                    best = cost;
+                    h->layout = l;
+                    h->TX = TX;
+                    h->TY = TY;
+                    h->ntx = ntx;
+                    h->nty = nty;
+                    h->nchunk = c;
+                }
+            }
+        });
+}
+
+// Tensor maps of the fused pass's boxes and the kernel's shared memory.
+tlm_status fusedMaps(fdtd_solver *h)
+{
+    const fdk::Dims &d = h->d;
+    auto encode = tlmi::tensorMapEncoder();
+    h->maps = std::make_unique<FdtdMaps>();
+    tlm_status st = TLM_OK;
+    withFusedLayout(h->layout, [&](auto L) {
+        using Layout = decltype(L);
+        for (int b = 0; b < 2; ++b)
+            for (int m = 0; m < 3; ++m)
+            {
+                const cuuint64_t dims[4] = { (cuuint64_t)d.px, (cuuint64_t)d.ny + 1, (cuuint64_t)d.nz + 1, 6 };
+                const cuuint64_t strides[3] = { (cuuint64_t)d.px * 4, (cuuint64_t)d.px * (d.ny + 1) * 4,
+                                                (cuuint64_t)h->P * 4 };
+                const cuuint32_t box[4] = { (cuuint32_t)Layout::W2, (cuuint32_t)(m == 2 ? Layout::H : Layout::H + 1), 1,
+                                            m == 0 ? 2u : m == 1 ? 1u : 3u };
+                const cuuint32_t es[4] = { 1, 1, 1, 1 };
+                if (encode(&h->maps->map[b][m], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->dBuf[b], dims, strides, box, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                    st = h->fail(TLM_ECUDA, "tensor map of a field buffer");
+            }
+        if (st == TLM_OK)
+            st = h->cuda(cudaFuncSetAttribute(fdk::fusedStepKernel<Layout>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              Layout::smemBytes),
+                         "cudaFuncSetAttribute(fusedStepKernel)");
+    });
+    return st;
+}
+
+// more: another step follows at once (its sources may go in with this step's tail)
+tlm_status launchStep(fdtd_solver *h, int n, bool more)
 {
     const fdk::Dims &d = h->d;
     fdk::Fields f;
     for (int c = 0; c < 3; ++c)
     {
-        f.E[c] = static_cast<float *>(h->dField[c]);
-        f.H[c] = static_cast<float *>(h->dField[3 + c]);
-        f.mE[c] = h->dMask[c];
+        f.E[c] = h->field(c);
+        f.H[c] = h->field(3 + c);
         f.ca[c] = h->dCa[c];
         f.cb[c] = h->dCb[c];
     }
-    const float sv = sourceValue(h, n);
+    f.cls = h->dCls;
+    f.tab = h->dTab;
     // 1. soft sources
-    if (h->nEdges)
-        fdk::injectKernel<<<(h->nEdges + 255) / 256, 256, 0, h->stream>>>(f, h->dEdge, h->dEdgeOff, h->dAmps,
-                                                                         h->nEdges, sv);
+    auto injectArgs = [&](float *E, int step) {
+        fdk::InjectArgs a;
+        for (int c = 0; c < 3; ++c) a.E[c] = E + c * h->P;
+        a.edge = h->dEdge;
+        a.off = h->dEdgeOff;
+        a.amps = h->dAmps;
+        a.nedges = h->nEdges;
+        a.sv = sourceValue(h, step);
+        return a;
+    };
+    const unsigned injectBlocks = (unsigned)((h->nEdges + 255) / 256);
+    if (h->nEdges && !h->injected)
+        fdk::injectKernel<<<injectBlocks, 256, 0, h->stream>>>(injectArgs(h->dBuf[h->cur], n));
+    h->injected = false;
     // 2. monitors
     SurfaceState &s = h->surf;
     const int nj = (int)s.jsCell.size(), nhuy = (int)s.huyCell.size();
@@ -926,7 +1516,8 @@ tlm_status launchStep(fdtd_solver *h, int n)
     a.planeN2 = n2;
     a.plane = static_cast<float *>(s.dPlane);
     const long long items = (long long)a.nports + a.nprobes + nj + (doDft ? nhuy : 0) + (doPlane ? (long long)n1 * n2 : 0);
-    if (items > 0) fdk::monitorKernel<<<(unsigned)((items + 255) / 256), 256, 0, h->stream>>>(a);
+    const bool fused = h->dBuf[1] != nullptr;
+    if (items > 0 && !fused) fdk::monitorKernel<<<(unsigned)((items + 255) / 256), 256, 0, h->stream>>>(a);
     if (doPlane)
     {
         s.planeValid = true;
@@ -938,9 +1529,62 @@ tlm_status launchStep(fdtd_solver *h, int n)
     if ((n & 15) == 0)
     {
         const double eta = (double)tlmh::eta0_f32();
-        fdk::energyPartialKernel<<<h->nEpart, 256, 0, h->stream>>>(f, h->len[0], h->len[1], h->len[2], h->len[3],
-                                                                  h->len[4], h->len[5], eta * eta, h->dEpart);
+        fdk::energyPartialKernel<<<h->nEpart, 256, 0, h->stream>>>(f, h->P, eta * eta, h->dEpart);
         fdk::energyFinalKernel<<<1, 256, 0, h->stream>>>(h->dEpart, h->nEpart, h->dEhist + n / 16);
+    }
+    // 3. H, 4. E and Mur
+    long long faceItems = 0;
+    for (int F = 0; F < 6; ++F) faceItems += (long long)h->mur.n1[F] * h->mur.n2[F];
+    const unsigned faceBlocks = (unsigned)((faceItems + 255) / 256);
+    if (fused)
+    {
+        fdk::FusedArgs fa;
+        fa.in = f;
+        fa.mapExy = h->maps->map[h->cur][0];
+        fa.mapEz = h->maps->map[h->cur][1];
+        fa.mapH = h->maps->map[h->cur][2];
+        fa.fault = h->dFault;
+        fa.out = h->dBuf[h->cur ^ 1];
+        fa.P = h->P;
+        fa.d = d;
+        fa.TX = h->TX;
+        fa.TY = h->TY;
+        fa.ntx = h->ntx;
+        fa.nty = h->nty;
+        fa.nchunk = h->nchunk;
+        fa.flags = h->dFlags;
+        fa.ch = h->ch;
+        fa.cb0 = h->cb0;
+        fa.neg_zero = -0.0f;
+        withFusedLayout(h->layout, [&](auto L) {
+            using Layout = decltype(L);
+            fdk::fusedStepKernel<Layout>
+                <<<(unsigned)(h->ntx * h->nty * h->nchunk), Layout::kThreads, Layout::smemBytes, h->stream>>>(fa);
+        });
+        fdk::TailArgs ta;
+        ta.oldE = h->dBuf[h->cur];
+        ta.newE = fa.out;
+        ta.P = h->P;
+        ta.mur = h->mur;
+        ta.mon = a;
+        ta.inj = injectArgs(fa.out, n + 1);
+        ta.murBlocks = faceBlocks;
+        ta.monBlocks = (unsigned)((items + 255) / 256);
+        h->injected = more && h->nEdges && h->edgesInside;
+        fdk::stepTailKernel<<<faceBlocks + ta.monBlocks + (h->injected ? injectBlocks : 0), 256, 0, h->stream>>>(ta);
+        h->cur ^= 1;
+    }
+    else
+    {
+        fdk::Box box = boxOf(d);
+        const unsigned grid = (box.total + 255) / 256;
+        fdk::updateHKernel<<<grid + faceBlocks, 256, 0, h->stream>>>(f, d, box, h->ch, h->mur, grid);
+        fdk::updateEKernel<<<grid, 256, 0, h->stream>>>(f, d, box);
+        long long aItems = 0, bItems = 0;
+        for (int F = 0; F < 3; ++F) aItems += (long long)h->mur.n1[F] * h->mur.n2[F];
+        for (int F = 3; F < 6; ++F) bItems += (long long)h->mur.n1[F] * h->mur.n2[F];
+        fdk::murApplyKernel<0><<<(unsigned)((aItems + 255) / 256), 256, 0, h->stream>>>(f, d, h->mur);
+        fdk::murApplyKernel<3><<<(unsigned)((bItems + 255) / 256), 256, 0, h->stream>>>(f, d, h->mur);
     }
     if (h->cfg.record_every > 0 && (n % h->cfg.record_every) == 0)
     {
@@ -972,22 +1616,6 @@ tlm_status launchStep(fdtd_solver *h, int n)
         s.frames.push_back(fr);
         s.framesUsed = need;
     }
-    // 3. H, 4. Mur snapshot, E, Mur
-    fdk::Box box;
-    box.total = (unsigned)((long long)(d.nx + 1) * (d.ny + 1) * (d.nz + 1));
-    box.divX = tlmk::makeFastDiv((unsigned)(d.nx + 1));
-    box.divY = tlmk::makeFastDiv((unsigned)(d.ny + 1));
-    const unsigned grid = (box.total + 255) / 256;
-    long long snapItems = 0;
-    for (int F = 0; F < 6; ++F) snapItems += (long long)h->mur.n1[F] * h->mur.n2[F];
-    const unsigned snapBlocks = (unsigned)((snapItems + 255) / 256);
-    fdk::updateHKernel<<<grid + snapBlocks, 256, 0, h->stream>>>(f, d, box, h->ch, h->mur, grid);
-    fdk::updateEKernel<<<grid, 256, 0, h->stream>>>(f, d, box, h->cb0);
-    long long aItems = 0, bItems = 0;
-    for (int F = 0; F < 3; ++F) aItems += (long long)h->mur.n1[F] * h->mur.n2[F];
-    for (int F = 3; F < 6; ++F) bItems += (long long)h->mur.n1[F] * h->mur.n2[F];
-    fdk::murApplyKernel<0><<<(unsigned)((aItems + 255) / 256), 256, 0, h->stream>>>(f, d, h->mur);
-    fdk::murApplyKernel<3><<<(unsigned)((bItems + 255) / 256), 256, 0, h->stream>>>(f, d, h->mur);
     return h->cuda(cudaGetLastError(), "FDTD step launch");
 }
 
@@ -1069,9 +1697,11 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     if (!(grid->dl > 0.0f)) return h->fail(TLM_EINVAL, "dl must be positive");
     const size_t n = (size_t)grid->nx * grid->ny * grid->nz;
     if (n_cells != n) return h->fail(TLM_EINVAL, "material map does not match the grid");
-    for (size_t c = 0; c < n; ++c)
-        if (mat[c] >= TLM_MAT_DIEL0 && (int)(mat[c] - TLM_MAT_DIEL0) >= n_table)
-            return h->fail(TLM_EINVAL, "material id without a table entry");
+    // the host copy of the map and its largest id in one vectorised pass
+    std::vector<uint8_t> hostMat(n);
+    const uint8_t maxId = tlmh::copy_max_u8(mat, hostMat.data(), n);
+    if (maxId >= TLM_MAT_DIEL0 && (int)(maxId - TLM_MAT_DIEL0) >= n_table)
+        return h->fail(TLM_EINVAL, "material id without a table entry");
     if (cfg->waveform < 0 || cfg->waveform > TLM_WAVE_TABLE) return h->fail(TLM_EINVAL, "unknown waveform");
     if (cfg->record_every < 0 || cfg->huy_offset < 0) return h->fail(TLM_EINVAL, "negative record_every or huy_offset");
     Guard gd(h->device);
@@ -1080,111 +1710,104 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     h->configured = false;
     h->g = *grid;
     h->cfg = *cfg;
-    h->mat.assign(mat, mat + n);
+    h->mat.swap(hostMat);
     h->table.assign(table, table + n_table);
-    h->d = fdk::Dims{ grid->nx, grid->ny, grid->nz };
+    h->d = fdk::Dims{ grid->nx, grid->ny, grid->nz, (grid->nx + 4) / 4 * 4 };
     const fdk::Dims &d = h->d;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
     h->dt = tlmh::fdtd_dt(grid->dl);
     h->cMur = tlmh::fdtd_cmur(h->dt, grid->dl);
     h->cb0 = tlmh::fdtd_cb0(h->dt, grid->dl);
     h->ch = tlmh::fdtd_ch(h->dt, grid->dl);
-    h->haveDiel = false;
-    for (size_t c = 0; c < n; ++c)
-        if (mat[c] >= TLM_MAT_DIEL0)
-        {
-            h->haveDiel = true;
-            break;
-        }
+    h->haveDiel = maxId >= TLM_MAT_DIEL0;
     h->len[0] = (long long)nx * (ny + 1) * (nz + 1);
     h->len[1] = (long long)(nx + 1) * ny * (nz + 1);
     h->len[2] = (long long)(nx + 1) * (ny + 1) * nz;
     h->len[3] = (long long)(nx + 1) * ny * nz;
     h->len[4] = (long long)nx * (ny + 1) * nz;
     h->len[5] = (long long)nx * ny * (nz + 1);
-    // per-edge classification (FdtdSolver.cpp:135-231)
-    std::vector<float> ca[3], cb[3];
-    for (int c = 0; c < 3; ++c)
+    h->P = (long long)d.px * (ny + 1) * (nz + 1);
+    h->cur = 0;
+    const size_t field = 6 * (size_t)h->P * 4, classes = (size_t)h->P * 4, mixed = h->haveDiel ? 6 * (size_t)h->P * 4 : 0;
+    const size_t need = field + classes + mixed, spare = (size_t)256 << 20;
+    const size_t avail = tlmi::poolAvailable(h->device);
+    if (need + spare > avail) return h->fail(TLM_ENOMEM, "grid needs " + std::to_string(need >> 20) + " MiB of HBM");
+    // a second field buffer for fused passes where it fits (their lane offsets
+    // within a plane are 32-bit); no_staging asks for the in-place sweeps
+    const bool fused = need + field + spare <= avail && !cfg->no_staging && (long long)d.px * (ny + 1) < (1LL << 30) &&
+                       tlmi::tensorMapEncoder() != nullptr;
+    for (int b = 0; b < (fused ? 2 : 1); ++b)
     {
-        h->hMask[c].assign((size_t)h->len[c], 1);
-        if (h->haveDiel)
-        {
-            ca[c].assign((size_t)h->len[c], 1.0f);
-            cb[c].assign((size_t)h->len[c], h->cb0);
-        }
-    }
-    const int ext[3][3] = { { nx, ny + 1, nz + 1 }, { nx + 1, ny, nz + 1 }, { nx + 1, ny + 1, nz } };
-    for (int axis = 0; axis < 3; ++axis)
-    {
-        const int t1 = axis == 0 ? 1 : 0, t2 = axis == 2 ? 1 : 2;
-        for (int k = 0; k < ext[axis][2]; ++k)
-            for (int j = 0; j < ext[axis][1]; ++j)
-                for (int i = 0; i < ext[axis][0]; ++i)
-                {
-                    const long long q = axis == 0 ? d.iEx(i, j, k) : axis == 1 ? d.iEy(i, j, k) : d.iEz(i, j, k);
-                    bool pec = false;
-                    float eAcc = 0.0f, sAcc = 0.0f;
-                    int cnt = 0;
-                    for (int d1 = -1; d1 <= 0; ++d1)
-                        for (int d2 = -1; d2 <= 0; ++d2)
-                        {
-                            int co[3] = { i, j, k };
-                            co[t1] += d1;
-                            co[t2] += d2;
-                            if (co[0] < 0 || co[1] < 0 || co[2] < 0 || co[0] >= nx || co[1] >= ny || co[2] >= nz)
-                                continue;
-                            const uint8_t m = mat[((size_t)co[2] * ny + co[1]) * nx + co[0]];
-                            float e1 = 1.0f, s1 = 0.0f;
-                            if (m == TLM_MAT_PEC)
-                                pec = true;
-                            else if (m >= TLM_MAT_DIEL0)
-                            {
-                                e1 += table[m - TLM_MAT_DIEL0].epsr - 1.0f;
-                                s1 += table[m - TLM_MAT_DIEL0].sigma;
-                            }
-                            eAcc += e1;
-                            sAcc += s1;
-                            ++cnt;
-                        }
-                    if (pec)
-                    {
-                        h->hMask[axis][(size_t)q] = 0;
-                        if (h->haveDiel)
-                        {
-                            ca[axis][(size_t)q] = 0.0f;
-                            cb[axis][(size_t)q] = 0.0f;
-                        }
-                        continue;
-                    }
-                    if (h->haveDiel && cnt > 0)
-                        tlmh::fdtd_edge_coef(eAcc, sAcc, cnt, h->dt, grid->dl, &ca[axis][(size_t)q],
-                                             &cb[axis][(size_t)q]);
-                }
-    }
-    size_t need = 0;
-    for (int c = 0; c < 6; ++c) need += (size_t)h->len[c] * 4;
-    for (int c = 0; c < 3; ++c) need += (size_t)h->len[c] * (h->haveDiel ? 9 : 1);
-    if (need + ((size_t)256 << 20) > tlmi::poolAvailable(h->device))
-        return h->fail(TLM_ENOMEM, "grid needs " + std::to_string(need >> 20) + " MiB of HBM");
-    for (int c = 0; c < 6; ++c)
-    {
-        FD_TRY(alloc(h, &h->dField[c], (size_t)h->len[c] * 4));
-        if (reinterpret_cast<uintptr_t>(h->dField[c]) & 15)  // the energy sweep reads 16-byte vectors
+        FD_TRY(alloc(h, &h->dBuf[b], field));
+        if (reinterpret_cast<uintptr_t>(h->dBuf[b]) & 15)  // vector loads
             return h->fail(TLM_ECUDA, "field allocation not 16-byte aligned");
-        FD_CU(h, cudaMemsetAsync(h->dField[c], 0, (size_t)h->len[c] * 4, h->stream));
+        FD_CU(h, cudaMemsetAsync(h->dBuf[b], 0, field, h->stream));
     }
-    for (int c = 0; c < 3; ++c)
-    {
-        FD_TRY(alloc(h, &h->dMask[c], (size_t)h->len[c]));
-        FD_CU(h, cudaMemcpyAsync(h->dMask[c], h->hMask[c].data(), (size_t)h->len[c], cudaMemcpyHostToDevice,
-                                 h->stream));
-        if (h->haveDiel)
+    FD_TRY(alloc(h, &h->dCls, classes));
+    FD_CU(h, cudaMemsetAsync(h->dCls, 0, classes, h->stream));
+    if (h->haveDiel)
+        for (int c = 0; c < 3; ++c)
         {
-            FD_TRY(alloc(h, &h->dCa[c], (size_t)h->len[c] * 4));
-            FD_TRY(alloc(h, &h->dCb[c], (size_t)h->len[c] * 4));
-            FD_CU(h, cudaMemcpyAsync(h->dCa[c], ca[c].data(), (size_t)h->len[c] * 4, cudaMemcpyHostToDevice, h->stream));
-            FD_CU(h, cudaMemcpyAsync(h->dCb[c], cb[c].data(), (size_t)h->len[c] * 4, cudaMemcpyHostToDevice, h->stream));
+            FD_TRY(alloc(h, &h->dCa[c], (size_t)h->P * 4));
+            FD_TRY(alloc(h, &h->dCb[c], (size_t)h->P * 4));
         }
+    // coefficients of the edges inside one material: the sums over four equal cells
+    std::vector<float2> tab(fdk::kEdgeClasses, make_float2(0.0f, 0.0f)), props(std::max(n_table, 1), make_float2(1.0f, 0.0f));
+    tab[fdk::kEdgeAir] = make_float2(1.0f, h->cb0);
+    for (int t = 0; t < n_table; ++t)
+    {
+        props[t] = make_float2(table[t].epsr, table[t].sigma);
+        const int id = t + TLM_MAT_DIEL0;
+        const float e1 = 1.0f + (table[t].epsr - 1.0f), s1 = table[t].sigma;
+        float e = 0.0f, sg = 0.0f;
+        for (int q = 0; q < 4; ++q)
+        {
+            e += e1;
+            sg += s1;
+        }
+        tlmh::fdtd_edge_coef(e, sg, 4, h->dt, grid->dl, &tab[id].x, &tab[id].y);
+    }
+    std::memset(&tab[fdk::kEdgeFirst], 0xff, (fdk::kEdgeClasses - fdk::kEdgeFirst) * sizeof(float2));
+    FD_TRY(alloc(h, &h->dTab, tab.size() * sizeof(float2)));
+    FD_CU(h, cudaMemcpyAsync(h->dTab, tab.data(), tab.size() * sizeof(float2), cudaMemcpyHostToDevice, h->stream));
+    {
+        uint8_t *dMat = nullptr;
+        float2 *dProps = nullptr;
+        FD_TRY(alloc(h, &dMat, n));
+        tlm_status st = alloc(h, &dProps, props.size() * sizeof(float2));
+        if (st == TLM_OK)
+        {
+            cudaError_t e = cudaMemcpyAsync(dMat, mat, n, cudaMemcpyHostToDevice, h->stream);
+            if (e == cudaSuccess)
+                e = cudaMemcpyAsync(dProps, props.data(), props.size() * sizeof(float2), cudaMemcpyHostToDevice,
+                                    h->stream);
+            if (e == cudaSuccess)
+            {
+                const fdk::Box box = boxOf(d);
+                fdk::edgeClassKernel<<<(box.total + 255) / 256, 256, 0, h->stream>>>(
+                    dMat, dProps, d, box, h->dt, grid->dl, tlmh::fdtd_eps0(), h->dCls,
+                    reinterpret_cast<unsigned long long *>(h->dTab), h->dCa[0], h->dCa[1], h->dCa[2],
+                    h->dCb[0], h->dCb[1], h->dCb[2]);
+                e = cudaGetLastError();
+            }
+            st = h->cuda(e, "edge classes");
+        }
+        release(h, dMat);
+        release(h, dProps);
+        FD_TRY(st);
+    }
+    if (fused)
+    {
+        int sms = 0;
+        FD_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+        chooseFused(h, sms);
+        FD_TRY(alloc(h, &h->dFault, sizeof(unsigned)));
+        FD_CU(h, cudaMemsetAsync(h->dFault, 0, sizeof(unsigned), h->stream));
+        FD_TRY(fusedMaps(h));
+        const size_t nf = (size_t)h->ntx * h->nty * (nz + 1);
+        FD_TRY(alloc(h, &h->dFlags, nf));
+        fdk::edgeFlagKernel<<<(unsigned)nf, 128, 0, h->stream>>>(h->dCls, d, h->TX, h->TY, h->ntx, h->dFlags);
+        FD_CU(h, cudaGetLastError());
     }
     // Mur planes: x faces (Ey, Ez), y faces (Ex, Ez), z faces (Ex, Ey)
     const int n1[6] = { ny, ny + 1, nx, nx + 1, nx, nx + 1 };
@@ -1209,6 +1832,7 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     tlmi::buildFaceLists(nx, ny, nz, grid->origin, grid->dl, mat, cfg->surface_monitors != 0, cfg->huy_offset,
                          h->surf);
     h->curStep = 0;
+    h->injected = false;
     h->prepared = false;
     h->configured = true;
     return TLM_OK;
@@ -1293,10 +1917,14 @@ tlm_status fdtd_step(fdtd_handle h, int n_steps)
     FD_TRY(ensureRecords(h, (long long)h->curStep + n_steps));
     for (int t = 0; t < n_steps; ++t)
     {
-        FD_TRY(launchStep(h, h->curStep));
+        FD_TRY(launchStep(h, h->curStep, t + 1 < n_steps));
         ++h->curStep;
     }
+    unsigned fault = 0;
+    if (h->dFault)
+        FD_CU(h, cudaMemcpyAsync(&fault, h->dFault, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
     FD_CU(h, cudaStreamSynchronize(h->stream));
+    if (fault) return h->fail(TLM_ECUDA, "a field plane's bulk copies never arrived");
     return TLM_OK;
 }
 
@@ -1335,9 +1963,18 @@ tlm_status fdtd_get_field(fdtd_handle h, int which, float *out, size_t cap, size
     if (!out) return TLM_OK;
     if (cap < (size_t)h->len[which]) return h->fail(TLM_EINVAL, "output smaller than the field");
     Guard gd(h->device);
-    FD_CU(h, cudaStreamSynchronize(h->stream));
-    FD_CU(h, cudaMemcpy(out, h->dField[which], (size_t)h->len[which] * 4, cudaMemcpyDeviceToHost));
-    return TLM_OK;
+    float *packed = nullptr;
+    FD_TRY(alloc(h, &packed, (size_t)h->len[which] * 4));
+    const int a = which % 3;  // E: one more entry on the axes other than a; H: one more on a
+    const int n0 = h->d.nx + ((which < 3) == (a != 0) ? 1 : 0), n1 = h->d.ny + ((which < 3) == (a != 1) ? 1 : 0);
+    fdk::packFieldKernel<<<tlmi::gridBlocksFor(h->len[which]), 256, 0, h->stream>>>(h->field(which), h->d, n0, n1,
+                                                                                  h->len[which], packed);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(out, packed, (size_t)h->len[which] * 4, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    release(h, packed);
+    return h->cuda(e, "field read-back");
 }
 
 tlm_status fdtd_get_probe(fdtd_handle h, int idx, float *ex, float *ey, float *ez, int cap, int *n)

@@ -100,6 +100,7 @@ float fdtd_dt(float dl) { return 0.99f * dl / (kC0 * std::sqrt(3.0f)); }
 float fdtd_cmur(float dt, float dl) { return (kC0 * dt - dl) / (kC0 * dt + dl); }
 float fdtd_cb0(float dt, float dl) { return dt / (kEps0 * dl); }
 float fdtd_ch(float dt, float dl) { return dt / (kMu0 * dl); }
+float fdtd_eps0() { return kEps0; }
 // Lossy-dielectric E coefficients of one edge from the sums of (1 + (epsr -
 // 1)) and sigma over its cnt in-grid neighbour cells (FdtdSolver.cpp:193-206).
 void fdtd_edge_coef(float eAcc, float sAcc, int cnt, float dt, float dl, float *ca, float *cb)

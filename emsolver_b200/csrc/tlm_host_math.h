@@ -19,6 +19,7 @@ float fdtd_dt(float dl);
 float fdtd_cmur(float dt, float dl);
 float fdtd_cb0(float dt, float dl);
 float fdtd_ch(float dt, float dl);
+float fdtd_eps0();
 void fdtd_edge_coef(float eAcc, float sAcc, int cnt, float dt, float dl, float *ca, float *cb);
 void dft_phase_f32(float f0, float dt, int n, float *c, float *s);
 void dft_phase_f64(float f0, double dt, int n, double *c, double *s);

@@ -5,6 +5,8 @@
 #include "tlm_b200.h"
 #include "tlm_device.cuh"
 
+#include <cuda.h>
+
 #include <atomic>
 #include <memory>
 #include <type_traits>
@@ -420,5 +422,11 @@ tlm_status launchSurface(tlm_solver *h, int n);
 cudaMemPool_t devicePool(int device);
 size_t poolAvailable(int device);
 bool poolCovers(int device, size_t bytes);
+// The driver's tensor-map encoder (null where the driver has none).
+using TensorMapEncoder = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                      const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
+                                      CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                                      CUtensorMapFloatOOBfill);
+TensorMapEncoder tensorMapEncoder();
 
 } // namespace tlmi

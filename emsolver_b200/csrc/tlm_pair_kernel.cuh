@@ -41,8 +41,6 @@
 
 #include "tlm_step_kernel.cuh"
 
-#include <cuda.h>
-
 namespace tlmk {
 
 
@@ -109,16 +107,6 @@ struct PairArgs
     unsigned long long stage_wait_ns;
     unsigned int *fault;
 };
-
-__device__ __forceinline__ void tmaBox4(unsigned dst, const CUtensorMap *map, int x, int y, int z, int s,
-                                        unsigned bar)
-{
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                 "[%0], [%1, {%2, %3, %4, %5}], [%6];"
-                 :
-                 : "r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(s), "r"(bar)
-                 : "memory");
-}
 
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
 {
@@ -334,7 +322,6 @@ __device__ __forceinline__ void negWhere(float2 &v, unsigned mask, float2 own)
     if (mask & 1u) v.x = -own.x;
     if (mask & 2u) v.y = -own.y;
 }
-__device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
 // DIEL: the grid has stub-loaded nodes.
 template <class L, bool DIEL>
 __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(const __grid_constant__ PairArgs a)

@@ -758,13 +758,9 @@ struct tlmi::PairPlan
 
 namespace tlmi {
 
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encodeTiled()
+TensorMapEncoder tensorMapEncoder()
 {
-    static EncodeTiled fn = []() -> EncodeTiled {
+    static TensorMapEncoder fn = []() -> TensorMapEncoder {
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
         if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) !=
@@ -774,7 +770,7 @@ EncodeTiled encodeTiled()
             cudaGetLastError();
             return nullptr;
         }
-        return reinterpret_cast<EncodeTiled>(p);
+        return reinterpret_cast<TensorMapEncoder>(p);
     }();
     return fn;
 }
@@ -786,7 +782,7 @@ tlm_status ensurePair(tlm_solver *h)
 {
     if (h->pairTried) return TLM_OK;
     h->pairTried = true;
-    EncodeTiled encode = encodeTiled();
+    TensorMapEncoder encode = tensorMapEncoder();
     if (!encode) return TLM_OK;
     if (h->dStub)
     {

@@ -18,6 +18,8 @@
 
 #include "tlm_device.cuh"
 
+#include <cuda.h>
+
 #include <climits>
 #include <type_traits>
 
@@ -299,6 +301,19 @@ __device__ __forceinline__ void bulkCopy(unsigned dst, const void *src, unsigned
                  : "r"(dst), "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
+
+// A box of a 4-dimensional tensor map into shared memory.
+__device__ __forceinline__ void tmaBox4(unsigned dst, const CUtensorMap *map, int x, int y, int z, int s,
+                                        unsigned bar)
+{
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                 "[%0], [%1, {%2, %3, %4, %5}], [%6];"
+                 :
+                 : "r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(s), "r"(bar)
+                 : "memory");
+}
+
+__device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
 
 // Interior tile (see kTileGeneral): the gather needs no PEC handling, so
 // every pulse load is issued before any material is read. On the outer faces

@@ -290,6 +290,14 @@ struct tlm_solver
     bool pairTried = false;
     unsigned *dPairFlags = nullptr;
     void *dStubAlt = nullptr;
+    // many steps per launch for small FP32 grids (tlm_resident_kernel.cuh):
+    // bricks of by x bz rows (resBy 0: none), the packets between them and the
+    // number of the last step sent, and the pairs' energy shares of a launch
+    bool resTried = false;
+    int resBy = 0, resBz = 0, resPairs = 0;
+    void *dResPack = nullptr;
+    unsigned resBase = 0;
+    double *dEpair = nullptr;
     std::vector<uint8_t> tileFlagsHost;
     void *dSamples = nullptr;
     double *dEpart = nullptr;

@@ -118,8 +118,35 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
     return r;
 }
 
-// Soft sources and monitor samples of the pair at node0 (the general tile
-// body's, for two nodes).
+// One source or monitor entry of a node of the pair (`second`: its second
+// node), as in the general tile body: a soft source adds to the node's incident
+// pulses, a monitor writes its node voltages and circulations to dst.
+__device__ __forceinline__ void pairSpecEntry(const SpecEntry &se, bool second, float sv, float *dst, unsigned live,
+                                              float2 (&inc)[12])
+{
+    if (se.kind == kInject)
+    {
+        const float qv = (0.5f * se.amp) * sv;
+#pragma unroll
+        for (int s = 0; s < 12; ++s)
+            if ((s >> 2) != se.arg && fieldOfSlot(s) == se.arg)
+            {
+                if (second) inc[s].y = inc[s].y + qv;
+                else inc[s].x = inc[s].x + qv;
+            }
+    }
+    else if (dst != nullptr)
+    {
+        const bool on = (live >> (second ? 1 : 0)) & 1u;
+        float v[12];
+#pragma unroll
+        for (int s = 0; s < 12; ++s) v[s] = on ? (second ? inc[s].y : inc[s].x) : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) dst[j] = nodeVoltage(v, j);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) dst[3 + k] = circulation(v, k);
+    }
+}
 __device__ __forceinline__ void pairSpec(const PairArgs &a, int step, long long node0, bool own, unsigned live,
                                          float2 (&inc)[12])
 {
@@ -133,30 +160,8 @@ __device__ __forceinline__ void pairSpec(const PairArgs &a, int step, long long 
     {
         const SpecEntry se = a.spec[e];
         if (se.node >= node0 + 2) break;
-        const bool second = se.node != node0;
-        if (se.kind == kInject)
-        {
-            const float qv = (0.5f * se.amp) * a.sv[step];
-#pragma unroll
-            for (int s = 0; s < 12; ++s)
-                if ((s >> 2) != se.arg && fieldOfSlot(s) == se.arg)
-                {
-                    if (second) inc[s].y = inc[s].y + qv;
-                    else inc[s].x = inc[s].x + qv;
-                }
-        }
-        else if (own)
-        {
-            const bool on = (live >> (second ? 1 : 0)) & 1u;
-            float v[12];
-#pragma unroll
-            for (int s = 0; s < 12; ++s) v[s] = on ? (second ? inc[s].y : inc[s].x) : 0.0f;
-            float *dst = a.samples[step] + (long long)se.arg * 6;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) dst[j] = nodeVoltage(v, j);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) dst[3 + k] = circulation(v, k);
-        }
+        pairSpecEntry(se, se.node != node0, a.sv[step], own ? a.samples[step] + (long long)se.arg * 6 : nullptr, live,
+                      inc);
     }
 }
 

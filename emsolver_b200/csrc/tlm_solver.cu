@@ -9,6 +9,7 @@
 #include "tlm_aux_kernels.cuh"
 #include "tlm_host_math.h"
 #include "tlm_pair_kernel.cuh"
+#include "tlm_resident_kernel.cuh"
 #include "tlm_step_kernel.cuh"
 
 #include <algorithm>
@@ -71,6 +72,10 @@ void freeMonitors(tlm_solver *h)
     h->pairTried = false;
     devFree(h, h->dPairFlags);
     devFree(h, h->dStubAlt);
+    h->resTried = false;
+    h->resBy = 0;
+    devFree(h, h->dResPack);
+    devFree(h, h->dEpair);
     devFree(h, h->dSamples);
     devFree(h, h->dEpart);
     devFree(h, h->dPortOff);
@@ -905,6 +910,158 @@ tlm_status launchPair(tlm_solver *h, int n, int i, long long eFirst)
     return TLM_OK;
 }
 
+// f(kernel, shared memory bytes) for bricks of `pairs` pairs.
+template <class F> void withResident(int pairs, bool diel, F &&f)
+{
+    if (pairs <= tlmk::kResidentThreads)
+        diel ? f(tlmk::residentKernel<1, true>, tlmk::ResidentLayout<1, true>::smemBytes)
+             : f(tlmk::residentKernel<1, false>, tlmk::ResidentLayout<1, false>::smemBytes);
+    else
+        diel ? f(tlmk::residentKernel<2, true>, tlmk::ResidentLayout<2, true>::smemBytes)
+             : f(tlmk::residentKernel<2, false>, tlmk::ResidentLayout<2, false>::smemBytes);
+}
+
+// Cut a small grid into bricks that fit the SMs' shared memory, once per
+// prepare: the fewest pairs per brick, then the fewest that need a neighbour's
+// pulses. Handles without a plan keep the other kernels.
+tlm_status ensureResident(tlm_solver *h)
+{
+    if (h->resTried) return TLM_OK;
+    h->resTried = true;
+    int sms = 0, coop = 0;
+    TLM_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    TLM_CU(h, cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
+    if (!coop) return TLM_OK;
+    const int hx = h->px / 2;
+    long long best = -1;
+    for (int by = 1; by <= h->ny && (long long)by * hx <= 2 * tlmk::kResidentThreads; ++by)
+        for (int bz = 1; bz <= h->nz && (long long)by * bz * hx <= 2 * tlmk::kResidentThreads; ++bz)
+        {
+            const long long blocks = (long long)((h->ny + by - 1) / by) * ((h->nz + bz - 1) / bz);
+            if (blocks > sms) continue;
+            // a brick of one row or plane between two others would need both
+            // neighbours' pulses per node (the last one ends at the wall)
+            if ((by < 2 && h->ny > 2) || (bz < 2 && h->nz > 2)) continue;
+            const int inner = std::max(by - 2, 0) * std::max(bz - 2, 0);
+            const long long cost = (long long)by * bz * hx * 1024 + (by * bz - inner);
+            if (best >= 0 && cost >= best) continue;
+            best = cost;
+            h->resBy = by;
+            h->resBz = bz;
+        }
+    if (best < 0) return TLM_OK;
+    h->resPairs = h->resBy * h->resBz * hx;
+    const int gy = (h->ny + h->resBy - 1) / h->resBy, gz = (h->nz + h->resBz - 1) / h->resBz;
+    cudaError_t e = cudaSuccess;
+    int perSm = 0;
+    withResident(h->resPairs, h->dStub != nullptr, [&](auto kernel, int smem) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, tlmk::kResidentThreads, smem);
+    });
+    // two parities of two directions per axis, zero: no step has the number 0
+    const size_t packs = 4 * (size_t)hx * ((size_t)gy * h->nz + (size_t)gz * h->ny) * sizeof(tlmk::ResPacket);
+    const size_t share = (size_t)(tlmk::kResidentSteps / 16 + 1) * (h->P / 2) * sizeof(double);
+    if (e != cudaSuccess || perSm < 1 || devAlloc(h, &h->dResPack, packs) != TLM_OK ||
+        devAlloc(h, &h->dEpair, share) != TLM_OK)
+    {
+        cudaGetLastError();
+        h->resBy = 0;
+        return TLM_OK;
+    }
+    TLM_CU(h, cudaMemsetAsync(h->dResPack, 0, packs, h->stream));
+    h->resBase = 0;
+    return TLM_OK;
+}
+
+bool residentAllowed(const tlm_solver *h)
+{
+    return h->storage == TLM_STORE_F32 && h->variant == 0 && !h->cfg.no_staging && !h->cfg.general_tiles &&
+           !h->ghostLo && !h->ghostHi && !surfaceActive(h) && !h->stateIncident &&
+           (!h->resTried || h->resBy > 0);
+}
+
+// Resident launches of one device follow one another (an event between them),
+// whatever their streams: two of them side by side could each hold SMs that the
+// other waits for.
+struct ResidentOrder
+{
+    std::mutex mu;
+    cudaEvent_t done = nullptr;
+};
+ResidentOrder &residentOrder(int device)
+{
+    static ResidentOrder order[64];
+    return order[device & 63];
+}
+
+// Steps n .. n+steps-1, the window's i-th to (i+steps-1)-th, in one launch.
+tlm_status launchResident(tlm_solver *h, int n, int i, int steps, long long eFirst)
+{
+    tlmk::ResidentArgs a;
+    a.buf[0] = static_cast<float *>(h->dPulses[h->curBuf]);
+    a.buf[1] = static_cast<float *>(h->dPulses[h->curBuf ^ 1]);
+    a.stub = static_cast<float *>(h->dStub);
+    a.mat = h->dMat;
+    a.yhat = static_cast<const float *>(h->dYhat);
+    a.ghat = static_cast<const float *>(h->dGhat);
+    a.ntable = (int)h->epsr.size();
+    a.P = h->P;
+    a.nx = h->nx;
+    a.ny = h->ny;
+    a.nz = h->nz;
+    a.px = h->px;
+    a.by = h->resBy;
+    a.bz = h->resBz;
+    a.gy = (h->ny + a.by - 1) / a.by;
+    a.gz = (h->nz + a.bz - 1) / a.bz;
+    a.rho = h->cfg.boundary_rho;
+    a.neg_zero = -0.0f;
+    a.spec = h->dSpec;
+    a.nspec = h->specCount;
+    a.samples = static_cast<float *>(h->dSamples) + (size_t)i * h->nsamp * 6;
+    a.nsamp = h->nsamp;
+    a.steps = steps;
+    a.first = n;
+    a.epair = h->dEpair;
+    a.packY = static_cast<tlmk::ResPacket *>(h->dResPack);
+    a.packZ = a.packY + 4 * (size_t)(h->px / 2) * a.gy * h->nz;
+    a.base = h->resBase;
+    a.fault = h->dFault;
+    for (int s = 0; s < steps; ++s) a.sv[s] = (float)sourceValue(h, n + s);
+    const unsigned blocks = (unsigned)(a.gy * a.gz);
+    cudaEvent_t after = nullptr;
+    TLM_TRY(timeLaunch(h, steps, &after));
+    {
+        ResidentOrder &order = residentOrder(h->device);
+        std::lock_guard<std::mutex> lk(order.mu);
+        if (order.done)
+            TLM_CU(h, cudaStreamWaitEvent(h->stream, order.done, 0));
+        else
+            TLM_CU(h, cudaEventCreateWithFlags(&order.done, cudaEventDisableTiming));
+        void *args[] = { &a };
+        cudaError_t e = cudaSuccess;
+        withResident(h->resPairs, h->dStub != nullptr, [&](auto kernel, int smem) {
+            e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kernel), dim3(blocks),
+                                            dim3(tlmk::kResidentThreads), args, (size_t)smem, h->stream);
+        });
+        TLM_CU(h, e);
+        TLM_CU(h, cudaEventRecord(order.done, h->stream));
+    }
+    const long long e0 = ((long long)n + 15) / 16 * 16;
+    if (e0 < (long long)n + steps)
+    {
+        const int ne = (int)(((long long)n + steps - 1 - e0) / 16 + 1);
+        tlmk::residentEnergy<<<dim3((unsigned)h->nblocks, (unsigned)ne), kBlock, 0, h->stream>>>(
+            h->dEpair, h->P / 2, h->dEpart + (size_t)((e0 - eFirst) / 16) * h->nblocks, h->nblocks);
+        TLM_CU(h, cudaGetLastError());
+    }
+    if (after) TLM_CU(h, cudaEventRecord(after, h->stream));
+    h->resBase += (unsigned)steps;
+    h->curBuf ^= steps & 1;
+    return TLM_OK;
+}
+
 template <class R> tlm_status launchEpilogue(tlm_solver *h, long long base, int w, long long eFirst,
                                              int nE)
 {
@@ -960,6 +1117,17 @@ tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stoppe
         for (int i = 0; i < w; ++i)
         {
             const int n = (int)(base + i);
+            if (i + 1 < w && residentAllowed(h))
+            {
+                TLM_TRY(ensureResident(h));
+                if (h->resBy > 0)
+                {
+                    const int steps = std::min(w - i, tlmk::kResidentSteps);
+                    TLM_TRY(launchResident(h, n, i, steps, eFirst));
+                    i += steps - 1;
+                    continue;
+                }
+            }
             if (i + 1 < w && pairAllowed(h))
             {
                 TLM_TRY(ensurePair(h));
@@ -2437,6 +2605,15 @@ tlm_status tlm_steps_per_pass(tlm_handle h, int *steps)
     DeviceGuard dg(h->device);
     TLM_TRY(prepare(h));
     *steps = 1;
+    if (residentAllowed(h))
+    {
+        TLM_TRY(ensureResident(h));
+        if (h->resBy > 0)
+        {
+            *steps = std::min(h->window, tlmk::kResidentSteps);
+            return TLM_OK;
+        }
+    }
     if (pairAllowed(h))
     {
         TLM_TRY(ensurePair(h));

@@ -551,7 +551,8 @@ class TlmSolver:
         return n.value
 
     def stepsPerPass(self) -> int:
-        """Steps per pass over the state (2 on large FP32 grids, else 1)."""
+        """Steps per pass over the state in global memory (2 on large FP32
+        grids, a launch window on small ones, else 1)."""
         n = C.c_int(0)
         self._c(self._L.tlm_steps_per_pass(self._h, C.byref(n)))
         return n.value

@@ -601,9 +601,11 @@ TLM_API tlm_status tlm_kernel_time(tlm_handle h, double *ms, long long *launches
  * interior tiles and the remaining tiles as two kernels; surface monitors add
  * one); the window epilogue every steps_per_launch steps is not counted. */
 TLM_API tlm_status tlm_step_launches(tlm_handle h, int *per_step);
-/* Steps the handle takes per pass over its state: 2 on large FP32 grids,
- * whose step kernel runs two steps per launch (an odd step at the end of a
- * launch window runs alone), else 1. */
+/* Steps the handle takes per pass over its state in global memory: a launch
+ * window (64 steps at most) on small FP32 grids, whose state stays in shared
+ * memory for a launch; 2 on large FP32 grids, whose step kernel runs two steps
+ * per launch; else 1. A single step at the end of a window runs alone, and the
+ * kernels of tlm_step_launches are those of single steps. */
 TLM_API tlm_status tlm_steps_per_pass(tlm_handle h, int *steps);
 
 #ifdef __cplusplus

@@ -8,18 +8,21 @@
 // cudaMalloc/cudaFree can cause. Such a caller keeps the pulse planes itself
 // and asks this entry point to advance them one step.
 //
-// The scratch the step needs is one FP64 energy partial per thread block and
-// a copy of the caller's dielectric tables padded to every possible material
-// id (ids past the caller's table read NaN there instead of reading past the
-// caller's buffer). They live in the file-scope arrays below, a fixed
-// 514 KiB of device memory that every GPU which loads this library holds
-// until the process exits. Host code must not pass an array's name to a
-// kernel (on the host that name is a stand-in, not a device address); the
-// device addresses are looked up once per device with cudaGetSymbolAddress.
+// One launch does the whole step: blocks walk over tiles of node pairs, build
+// the stub table of the caller's materials in shared memory (ids past the
+// caller's n_diel entries read NaN there instead of reading past the caller's
+// buffers), and the last block to finish adds up the blocks' energies in a
+// fixed order. The only scratch, an FP64 partial per block and the count of
+// finished blocks, lives in the file-scope arrays below, a fixed 16 KiB of
+// device memory that every GPU which loads this library holds until the
+// process exits. Host code must not pass an array's name to a kernel (on the
+// host that name is a stand-in, not a device address); the device addresses
+// are looked up once per device with cudaGetSymbolAddress.
 #include "tlm_b200.h"
 
-#include "tlm_step_kernel.cuh"
+#include "tlm_pair_kernel.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -27,15 +30,12 @@
 // tlm_last_error(NULL).
 void tlmSetThreadError(const std::string &m);
 
-// Scratch: one energy partial per step-kernel block. 65,536 blocks of 256
-// threads x 4 nodes bound the grid at 67,108,864 padded nodes.
-constexpr int kNoAllocMaxBlocks = 65536;
-constexpr int kNoAllocV = 4;  // nodes per thread: 65536 blocks x 256 x 4 = 67,108,864 nodes
+// The grid is limited to 67,108,864 padded nodes (2^25 pairs).
+constexpr long long kNoAllocMaxNodes = 67108864;
+constexpr int kNoAllocMaxBlocks = 2048;
 static __device__ __align__(256) double g_noallocPartials[kNoAllocMaxBlocks];
-// Dielectric tables (yhat, ghat) for every material id 2..255: the caller's
-// n_diel entries, then NaN.
+static __device__ __align__(256) unsigned g_noallocDone;
 constexpr int kNoAllocTable = 256 - tlmk::kDiel0;
-static __device__ __align__(256) float g_noallocTables[2 * kNoAllocTable];
 // Bounds-check record of the checked library build (cleared before every
 // step, read back after it there); the regular build never writes it.
 static __device__ __align__(256) unsigned g_noallocFault;
@@ -48,7 +48,7 @@ std::mutex g_noallocMutex;
 struct NoAllocScratch
 {
     double *partials = nullptr;
-    float *tables = nullptr;
+    unsigned *done = nullptr;
     unsigned *fault = nullptr;
 };
 NoAllocScratch g_noallocAddr[kMaxDevices];
@@ -59,26 +59,175 @@ tlm_status noallocFail(tlm_status s, const std::string &m)
     return s;
 }
 
-// Fixed-order sum of the block partials into the caller's output.
-__global__ void __launch_bounds__(256) noallocEnergyReduce(const double *partials, int n, double *out)
+struct PlanesArgs
 {
-    __shared__ double red[tlmk::kBlock / 32];
-    double s = 0.0;
-    for (int b = threadIdx.x; b < n; b += blockDim.x) s += partials[b];
-    const double tot = tlmk::blockSumDouble(s, red);
-    if (threadIdx.x == 0) *out = tot;
-}
+    const float *in;
+    float *out, *stub;
+    const uint8_t *mat;
+    const float *yhat, *ghat;
+    int ntable;
+    int nx, ny, nz, px, hx;  // hx: pairs per row
+    long long P;
+    unsigned npairs;
+    tlmk::FastDiv divH, divY;  // by hx and by ny
+    float rho, neg_zero;
+    double *partials, *energy;
+    unsigned *done, *fault;
+};
 
-// The caller's yhat/ghat (n entries each) into the padded static tables;
-// the entries of ids past the caller's table are NaN, so a node with such an
-// id steps to NaN pulses instead of reading past the caller's buffers.
-__global__ void __launch_bounds__(kNoAllocTable) noallocTables(const float *yhat, const float *ghat, int n,
-                                                               float *tables)
+// One step, a pair of nodes per thread at a time, the arithmetic of the general
+// tile body (DIEL: with the caller's stubs). Every load of a pair that does not depend on its material
+// is issued before the first use; a pair next to PEC (rare) then loads the own
+// pulses it reflects. What bounds it at a few hundred thousand nodes is that
+// latency: 93x80x71 nodes (the caller's energy included) took three launches
+// and 34.6 us with the general tile body, four nodes per thread.
+template <bool INCIDENT, bool DIEL> __global__ void __launch_bounds__(256, 4) planesStepKernel(const PlanesArgs a)
 {
-    const int t = threadIdx.x;
-    if (t >= kNoAllocTable) return;
-    tables[t] = t < n ? yhat[t] : __int_as_float(0x7fc00000);
-    tables[kNoAllocTable + t] = t < n ? ghat[t] : __int_as_float(0x7fc00000);
+    using namespace tlmk;
+    __shared__ float tab[768];
+    __shared__ double red[8];
+    __shared__ bool lastBlock;
+    if constexpr (DIEL)
+    {
+        for (int m = threadIdx.x; m < 256; m += 256)
+        {
+            const float nan = __int_as_float(0x7fc00000);
+            const float yh = m < kDiel0 ? -0.0f : m - kDiel0 < a.ntable ? a.yhat[m - kDiel0] : nan;
+            const float gh = m < kDiel0 ? 0.0f : m - kDiel0 < a.ntable ? a.ghat[m - kDiel0] : nan;
+            const float den = (4.0f + yh) + gh;
+            tab[m] = yh;
+            tab[256 + m] = -den;
+            tab[512 + m] = __frcp_rn(den);
+        }
+        __syncthreads();
+    }
+    const long long P = a.P, sz = (long long)a.px * a.ny;
+    const float2 z = splat2(a.neg_zero), rho = splat2(a.rho);
+    double en = 0.0;
+    for (unsigned q = blockIdx.x * 256u + threadIdx.x; q < a.npairs; q += gridDim.x * 256u)
+    {
+        const unsigned row = fastDiv(q, a.divH);
+        const int x = 2 * (int)(q - row * (unsigned)a.hx);
+        const unsigned k = fastDiv(row, a.divY);
+        const int j = (int)(row - k * (unsigned)a.ny);
+        const long long n0 = 2LL * q;
+        if (!TLM_GUARD(n0, P - 1, 1)) continue;
+        const bool ylo = j == 0, yhi = j == a.ny - 1, zlo = k == 0, zhi = (int)k == a.nz - 1;
+        float2 inc[12];
+        unsigned pec = 0;  // two bits per face: -x +x -y +y -z +z
+        unsigned ids = *reinterpret_cast<const unsigned short *>(a.mat + n0);
+        if constexpr (INCIDENT)
+        {
+#pragma unroll
+            for (int s = 0; s < 12; ++s) inc[s] = ld2(a.in + s * P + n0);
+        }
+        else
+        {
+            const unsigned own = ((ids & 255u) == kPec ? 1u : 0u) | ((ids >> 8) == kPec ? 2u : 0u);
+            const bool prev = x > 0, next = x + 2 < a.nx;
+            const unsigned mp = prev ? a.mat[n0 - 1] : 0u, mn = next ? a.mat[n0 + 2] : 0u;
+            const unsigned mym = ylo ? 0u : pecPair(a.mat + n0 - a.px), myp = yhi ? 0u : pecPair(a.mat + n0 + a.px);
+            const unsigned mzm = zlo ? 0u : pecPair(a.mat + n0 - sz), mzp = zhi ? 0u : pecPair(a.mat + n0 + sz);
+            float2 ox[4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) ox[s] = ld2(a.in + s * P + n0);
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+            {
+                const float p = prev ? a.in[(2 + t) * P + n0 - 1] : 0.0f, n = next ? a.in[t * P + n0 + 2] : 0.0f;
+                inc[t] = make_float2(p, ox[2 + t].x);
+                inc[2 + t] = make_float2(ox[t].y, n);
+                inc[4 + t] = ld2(a.in + (ylo ? (4 + t) * P + n0 : (6 + t) * P + n0 - a.px));
+                inc[6 + t] = ld2(a.in + (yhi ? (6 + t) * P + n0 : (4 + t) * P + n0 + a.px));
+                inc[8 + t] = ld2(a.in + (zlo ? (8 + t) * P + n0 : (10 + t) * P + n0 - sz));
+                inc[10 + t] = ld2(a.in + (zhi ? (10 + t) * P + n0 : (8 + t) * P + n0 + sz));
+            }
+            pec = ((own << 1) & 2u) | (mp == kPec ? 1u : 0u);
+            pec |= ((x + 1 < a.nx ? own >> 1 : 0u) | (mn == kPec ? 2u : 0u)) << 2;
+            pec |= mym << 4 | myp << 6 | mzm << 8 | mzp << 10;
+            if (pec)
+            {
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+                {
+                    negWhere(inc[t], pec & 3u, ox[t]);
+                    negWhere(inc[2 + t], (pec >> 2) & 3u, ox[2 + t]);
+                    if ((pec >> 4) & 3u) negWhere(inc[4 + t], (pec >> 4) & 3u, ld2(a.in + (4 + t) * P + n0));
+                    if ((pec >> 6) & 3u) negWhere(inc[6 + t], (pec >> 6) & 3u, ld2(a.in + (6 + t) * P + n0));
+                    if ((pec >> 8) & 3u) negWhere(inc[8 + t], (pec >> 8) & 3u, ld2(a.in + (8 + t) * P + n0));
+                    if ((pec >> 10) & 3u) negWhere(inc[10 + t], (pec >> 10) & 3u, ld2(a.in + (10 + t) * P + n0));
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+            {
+                if (x == 0) inc[t].x = a.rho * ox[t].x;
+                if (x == a.nx - 1) inc[2 + t].x = a.rho * ox[2 + t].x;
+                if (x + 1 == a.nx - 1) inc[2 + t].y = a.rho * ox[2 + t].y;
+                if (ylo) inc[4 + t] = mul2(inc[4 + t], rho, z);
+                if (yhi) inc[6 + t] = mul2(inc[6 + t], rho, z);
+                if (zlo) inc[8 + t] = mul2(inc[8 + t], rho, z);
+                if (zhi) inc[10 + t] = mul2(inc[10 + t], rho, z);
+            }
+        }
+        unsigned word = matWord(ids, x + 1 < a.nx ? 0u : x < a.nx ? 2u : 3u);
+        if (a.energy != nullptr) en += pairEnergy(inc, 3u & ~(word >> 18));
+        float2 o[12];
+        if (DIEL && (word & kMatDiel))
+        {
+            float2 vs[3];
+#pragma unroll
+            for (int t = 0; t < 3; ++t) vs[t] = ld2(a.stub + t * P + n0);
+            pairScatterStub(tab, inc, vs, word, z, o);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) *reinterpret_cast<float2 *>(a.stub + t * P + n0) = vs[t];
+        }
+        else
+        {
+            // (without any table an id of a dielectric steps to NaN)
+            scatterAir2(inc, o, z);
+            if (!DIEL && (word & kMatDiel))
+            {
+#pragma unroll
+                for (int s = 0; s < 12; ++s)
+                {
+                    if (word & (1u << 16)) o[s].x = __int_as_float(0x7fc00000);
+                    if (word & (2u << 16)) o[s].y = __int_as_float(0x7fc00000);
+                }
+            }
+        }
+        if (word & kMatDead)
+        {
+#pragma unroll
+            for (int s = 0; s < 12; ++s)
+            {
+                if (word & (1u << 18)) o[s].x = 0.0f;
+                if (word & (2u << 18)) o[s].y = 0.0f;
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 12; ++s) *reinterpret_cast<float2 *>(a.out + s * P + n0) = o[s];
+    }
+    if (a.energy == nullptr) return;
+    const double tot = blockSumDouble(en, red);
+    if (threadIdx.x == 0)
+    {
+        a.partials[blockIdx.x] = tot;
+        __threadfence();
+        lastBlock = atomicAdd(a.done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!lastBlock) return;
+    __threadfence();
+    double s = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += 256) s += __ldcg(a.partials + b);
+    __syncthreads();
+    const double all = blockSumDouble(s, red);
+    if (threadIdx.x == 0)
+    {
+        *a.energy = all;
+        *a.done = 0;
+    }
 }
 
 // Device addresses of the scratch arrays for the current device, looked up
@@ -99,7 +248,7 @@ tlm_status scratchForCurrentDevice(NoAllocScratch *out)
     {
         void *p = nullptr, *t = nullptr, *f = nullptr;
         e = cudaGetSymbolAddress(&p, g_noallocPartials);
-        if (e == cudaSuccess) e = cudaGetSymbolAddress(&t, g_noallocTables);
+        if (e == cudaSuccess) e = cudaGetSymbolAddress(&t, g_noallocDone);
         if (e == cudaSuccess) e = cudaGetSymbolAddress(&f, g_noallocFault);
         if (e != cudaSuccess || !p || !t || !f)
         {
@@ -107,7 +256,7 @@ tlm_status scratchForCurrentDevice(NoAllocScratch *out)
             return noallocFail(TLM_ECUDA, std::string("cudaGetSymbolAddress of the scratch arrays: ") +
                                               cudaGetErrorString(e));
         }
-        sc.tables = static_cast<float *>(t);
+        sc.done = static_cast<unsigned *>(t);
         sc.fault = static_cast<unsigned *>(f);
         sc.partials = static_cast<double *>(p);
     }
@@ -139,8 +288,7 @@ tlm_status tlm_step_planes_noalloc(const float *in_planes, float *out_planes, fl
     if (!aligned16(in_planes) || !aligned16(out_planes) || (stubs && !aligned16(stubs)) ||
         ((uintptr_t)mat & 3u))
         return noallocFail(TLM_EINVAL, "planes must be 16-byte aligned, the material map 4-byte aligned");
-    constexpr int V = kNoAllocV;
-    constexpr long long kMaxNodes = (long long)kNoAllocMaxBlocks * tlmk::kBlock * V;
+    constexpr long long kMaxNodes = kNoAllocMaxNodes;
     // the plane size grows one factor at a time, each partial product
     // checked against the limit, so nothing overflows
     const long long px = ((long long)nx + tlmk::kPadX - 1) / tlmk::kPadX * tlmk::kPadX;
@@ -150,64 +298,55 @@ tlm_status tlm_step_planes_noalloc(const float *in_planes, float *out_planes, fl
         return noallocFail(TLM_EINVAL,
                            "grid has more than " + std::to_string(kMaxNodes) + " padded nodes; the no-allocation "
                            "step handles at most " + std::to_string(kMaxNodes));
-    const long long nq = px / V;
-    const long long nquads = nq * ny * nz;
-    const long long nblocks = (nquads + tlmk::kBlock - 1) / tlmk::kBlock;
-    if (nblocks <= 0 || nblocks > kNoAllocMaxBlocks)
-        return noallocFail(TLM_EINVAL, "grid block count out of range");
     NoAllocScratch sc;
     tlm_status st = scratchForCurrentDevice(&sc);
     if (st != TLM_OK) return st;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    noallocTables<<<1, kNoAllocTable, 0, s>>>(yhat, ghat, n_diel, sc.tables);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = cudaSuccess;
 #ifdef TLM_CHECKED
     if (e == cudaSuccess) e = cudaMemsetAsync(sc.fault, 0, sizeof(unsigned), s);
 #endif
     if (e != cudaSuccess)
         return noallocFail(TLM_ECUDA, std::string("no-allocation step set-up: ") + cudaGetErrorString(e));
 
-    tlmk::StepArgs<float> a;
+    PlanesArgs a;
     a.in = in_planes;
     a.out = out_planes;
     a.stub = stubs;
     a.mat = mat;
-    a.yhat = sc.tables;
-    a.ghat = sc.tables + kNoAllocTable;
-    a.P = P;
-    a.nquads = nquads;
+    a.yhat = yhat;
+    a.ghat = ghat;
+    a.ntable = n_diel;
     a.nx = nx;
     a.ny = ny;
     a.nz = nz;
     a.px = (int)px;
-    a.nq = (int)nq;
-    a.div_nq = tlmk::makeFastDiv((unsigned)nq);
-    a.div_ny = tlmk::makeFastDiv((unsigned)ny);
+    a.hx = (int)(px / 2);
+    a.P = P;
+    a.npairs = (unsigned)(P / 2);
+    a.divH = tlmk::makeFastDiv((unsigned)a.hx);
+    a.divY = tlmk::makeFastDiv((unsigned)ny);
     a.rho = rho;
-    a.scale = 1.0f;
-    a.inv_scale = 1.0f;
-    a.tile_begin = nullptr;
-    a.spec = nullptr;
-    a.tile_flags = nullptr;  // every tile takes the general body
     a.neg_zero = -0.0f;
-    a.sv = 0.0f;
-    a.samples = nullptr;
-    a.epart = energy_out ? sc.partials : nullptr;
-    a.e_lo = 0;
-    a.e_hi = LLONG_MAX;
+    a.partials = sc.partials;
+    a.energy = energy_out;
+    a.done = sc.done;
     a.fault = sc.fault;
-    a.stage_wait_ns = tlmk::kStageWaitNs;
+    // four resident blocks per SM walk over the tiles of large grids
+    const unsigned blocks = std::min((a.npairs + 255u) / 256u, 148u * 4u);
+    static_assert(148 * 4 <= kNoAllocMaxBlocks, "a partial per block");
     if (input_is_incident)
-        tlmk::stepKernelShaped<float, kNoAllocV, 3, true, false><<<(unsigned)nblocks, tlmk::kBlock, 0, s>>>(a);
-    else
-        tlmk::stepKernelShaped<float, kNoAllocV, 3, false, false><<<(unsigned)nblocks, tlmk::kBlock, 0, s>>>(a);
-    e = cudaGetLastError();
-    if (e == cudaSuccess && energy_out)
     {
-        noallocEnergyReduce<<<1, 256, 0, s>>>(sc.partials, (int)nblocks, energy_out);
-        e = cudaGetLastError();
+        if (stubs) planesStepKernel<true, true><<<blocks, 256, 0, s>>>(a);
+        else planesStepKernel<true, false><<<blocks, 256, 0, s>>>(a);
     }
+    else
+    {
+        if (stubs) planesStepKernel<false, true><<<blocks, 256, 0, s>>>(a);
+        else planesStepKernel<false, false><<<blocks, 256, 0, s>>>(a);
+    }
+    e = cudaGetLastError();
     if (e != cudaSuccess)
         return noallocFail(TLM_ECUDA, std::string("no-allocation step launch: ") + cudaGetErrorString(e));
 #ifdef TLM_CHECKED

@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
 // Flags of every (column, plane): PEC and dielectric nodes from the padded
 // material map (one block per column and plane; PEC within one node of the
 // grown column, the planes below and above included).
-__global__ void __launch_bounds__(128) pairMaterialFlags(const uint8_t *__restrict__ mat, int nx, int ny, int nz, int px,
+inline __global__ void __launch_bounds__(128) pairMaterialFlags(const uint8_t *__restrict__ mat, int nx, int ny, int nz, int px,
                                                          PairShape g, unsigned *__restrict__ flags)
 {
     const int k = blockIdx.x % nz, col = blockIdx.x / nz;
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(128) pairMaterialFlags(const uint8_t *__restri
 }
 
 // ... and the columns whose grown area holds a source or monitor node.
-__global__ void __launch_bounds__(128) pairSpecFlags(const SpecEntry *__restrict__ spec, int n, int ny, int nz, int px,
+inline __global__ void __launch_bounds__(128) pairSpecFlags(const SpecEntry *__restrict__ spec, int n, int ny, int nz, int px,
                                                      PairShape g, unsigned *__restrict__ flags)
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;

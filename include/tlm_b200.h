@@ -548,23 +548,21 @@ TLM_API tlm_status tlm_get_halo_stream(tlm_handle h, void **stream);
  * stubs: 3 planes read and written on dielectric nodes. yhat/ghat: n_diel
  * entries, one per dielectric id (id - 2); with n_diel > 0 stubs, yhat and
  * ghat must all be given (else TLM_EINVAL), with n_diel = 0 they may be NULL.
- * The tables are copied into a static table of all 254 dielectric ids whose
- * entries past n_diel are NaN: a node whose id is 2 + n_diel or more steps to
- * NaN pulses, and nothing past the caller's buffers is read. No sources or
- * monitors.
+ * A node whose id is 2 + n_diel or more steps to NaN pulses, and nothing past
+ * the caller's buffers is read. No sources or monitors.
  * energy_out (NULL to skip): the FP64 sum of the squares of all incident
  * link pulses of this step. Planes 16-byte aligned, mat 4-byte aligned.
  * Work is queued on `stream` (a cudaStream_t, NULL = default stream).
  *
  * Limits and sharing: its only scratch, one FP64 energy partial per thread
- * block and the padded dielectric table, is a fixed 514 KiB of static device
+ * block and a count of finished blocks, is a fixed 16 KiB of static device
  * arrays that every GPU loading this library holds until the process exits;
  * grids above 67,108,864 padded nodes are rejected with TLM_EINVAL. The
  * first call on a device looks up those arrays' device addresses
  * (cudaGetSymbolAddress); make that first call before any stream capture.
  * Every call shares the arrays, so calls that overlap on the GPU (other
- * streams, other threads) race: serialise them. Each call rewrites the table
- * and the partials it uses; nothing needs clearing. The bounds-checked build
+ * streams, other threads) race: serialise them. Each call rewrites the
+ * partials it uses and leaves the count at zero; nothing needs clearing. The bounds-checked build
  * of the library (libtlm_b200_checked.so) waits for the step and returns
  * TLM_ECUDA if any index fell outside its buffer.
  * Errors: status code, message in tlm_last_error(NULL). */

@@ -188,7 +188,9 @@ struct SurfaceState
 // The plan of two-step passes (tlm_pair_kernel.cuh; defined in tlm_solver.cu).
 struct PairPlan;
 
-// Two-step passes serve FP32 grids from this many padded nodes on.
+// Two-step passes serve FP32 grids from this many padded nodes on (at 104^3,
+// 1.12 M nodes, 23-27 us per step against 25-27 with single steps; at 96^3 the
+// two are even, at 88^3 14.2 against 13.3 us).
 constexpr long long kPairMinNodes = 1LL << 20;
 inline bool pairStorage(int storage, long long P) { return storage == TLM_STORE_F32 && P >= kPairMinNodes; }
 } // namespace tlmi
@@ -289,6 +291,8 @@ struct tlm_solver
     std::shared_ptr<tlmi::PairPlan> pair;
     bool pairTried = false;
     unsigned *dPairFlags = nullptr;
+    unsigned *dPairWord = nullptr;       // material word of every node pair
+    int *dSpecRow = nullptr;             // first entry of dSpec in every row of nodes
     void *dStubAlt = nullptr;
     // many steps per launch for small FP32 grids (tlm_resident_kernel.cuh):
     // bricks of by x bz rows (resBy 0: none), the packets between them and the

@@ -15,8 +15,9 @@
 // So two steps cost one read and one write of the state (plus the ring, which
 // mostly hits L2). The arithmetic of a node is that of the interior and
 // general tile bodies (tlm_step_kernel.cuh), in their order, so pulses, stubs
-// and monitor samples are bitwise those of two single steps; the energy is an
-// FP64 sum in another order.
+// and monitor samples are bitwise those of two single steps. An energy step
+// leaves every pair's FP64 share in `epair`, and pairEnergySums adds those up in
+// the order of the single-step kernels' tiles: the energies are bitwise too.
 //
 // The input planes come in by tensor-map bulk copies (TMA), five boxes per
 // plane: x slots at the column, y slots with one more row on either side (the
@@ -30,13 +31,14 @@
 // double-buffered like the pulses.
 //
 // Measured on a B200, one step: 192^3 air 111 -> 66 us, the 192^3 heterogeneous
-// grid 127 -> 96 us (its early steps 130 -> 104), 128^3 heterogeneous 48 -> 36
-// us, the 384x384x256 dipole 566 -> 340 us. What bounds it: air columns move
-// 0.64 GB a pass at 4.9 TB/s, 0.75 of the copy bandwidth, with 16 warps per SM
-// coupled by a barrier per plane; stub-loaded columns issue about 570
-// instructions per warp and plane instead of 330. Two blocks of 256 threads
+// grid 127 -> 98 us, 128^3 heterogeneous 48 -> 36 us, a 384x384x256 dipole 566
+// -> 340 us and beside a stub-loaded slab 645 -> 440 us. What bounds it: air
+// columns move 0.64 GB a pass at 4.9 TB/s, 0.75 of the copy bandwidth, with 16
+// warps per SM coupled by a barrier per plane; stub-loaded columns issue about
+// 570 instructions per warp and plane instead of 330. Two blocks of 256 threads
 // per SM (smaller columns, larger rings) measured 77 against 66 us in air, a
-// 640-thread block 80 us (spills).
+// 640-thread block 80 us (spills), a second walk without stub code for the
+// blocks of a stub-loaded grid that hold none 125 against 98 us (spills).
 #pragma once
 
 #include "tlm_step_kernel.cuh"
@@ -90,19 +92,18 @@ struct PairArgs
     float *out;
     const float *stubIn;
     float *stubOut;
-    const uint8_t *mat;
     const float *yhat, *ghat;
     int ntable;
     const unsigned *flags;         // [column][nz]
     long long P;
     int nx, ny, nz, px;
     float rho;
+    const unsigned *words;         // material word of every pair, with its PEC faces
     const SpecEntry *spec;
-    int nspec;
+    const int *specRow;            // first entry of every row of nodes, and their number after the last
     float sv[2];                   // source values of the two steps
     float *samples[2];             // [nsamp][6]
-    double *epart[2];              // energy partials (nullptr: no energy step)
-    int nepart;                    // partials the epilogue sums per energy step
+    double *epair[2];              // FP64 energy share of every pair (nullptr: no energy step)
     float neg_zero;
     unsigned long long stage_wait_ns;
     unsigned int *fault;
@@ -147,26 +148,29 @@ __device__ __forceinline__ void pairSpecEntry(const SpecEntry &se, bool second, 
         for (int k = 0; k < 3; ++k) dst[3 + k] = circulation(v, k);
     }
 }
-__device__ __forceinline__ void pairSpec(const PairArgs &a, int step, long long node0, bool own, unsigned live,
-                                         float2 (&inc)[12])
+__device__ __forceinline__ void pairSpec(const PairArgs &a, int step, long long row, long long node0, bool own,
+                                         unsigned live, float2 (&inc)[12])
 {
-    int lo = 0, hi = a.nspec;
-    while (lo < hi)
+    int lo = a.specRow[row];
+    const int end = a.specRow[row + 1];
+    for (int hi = end; hi - lo > 4;)  // rows that a plane wave fills
     {
         const int mid = (lo + hi) >> 1;
-        if (a.spec[mid].node < node0) lo = mid + 1; else hi = mid;
+        if (a.spec[mid].node < node0) lo = mid; else hi = mid;
     }
-    for (int e = lo; e < a.nspec; ++e)
+    for (int e = lo; e < end; ++e)
     {
         const SpecEntry se = a.spec[e];
         if (se.node >= node0 + 2) break;
+        if (se.node < node0) continue;
         pairSpecEntry(se, se.node != node0, a.sv[step], own ? a.samples[step] + (long long)se.arg * 6 : nullptr, live,
                       inc);
     }
 }
 
 // The material word of a pair: the two ids, which nodes are stub-loaded, and
-// which are dead (PEC, row padding or outside the grid).
+// which are dead (PEC, row padding or outside the grid); the twelve bits above
+// hold its PEC faces.
 enum : unsigned { kMatDiel = 3u << 16, kMatDead = 3u << 18 };
 __device__ __forceinline__ unsigned matWord(unsigned ids, unsigned dead)
 {
@@ -226,6 +230,11 @@ __device__ __forceinline__ void pairScatterStub(const float *tab, const float2 (
     }
     if (lo > 0x1p-100f && hi < 0x1p120f)
         divByTable(num, nden, rcp, z, Vn);
+    else if (hi == 0.0f)
+    {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) Vn[j] = num[j];
+    }
     else if (hi < 0x1p40f)
     {
         // distance of each scaled quotient from the value it scales back to
@@ -295,32 +304,28 @@ __device__ __forceinline__ double pairEnergy(const float2 (&inc)[12], unsigned l
     return e;
 }
 
-// PEC masks (2 bits, one per node of the pair) of the six neighbours of the
-// pair at (x, j, k); a neighbour outside the grid counts as none (the wall
-// comes first, as in the general tile body).
-struct PairPec
-{
-    unsigned xm, xp, ym, yp, zm, zp;
-};
 __device__ __forceinline__ unsigned pecPair(const uint8_t *m)
 {
     const unsigned v = *reinterpret_cast<const unsigned short *>(m);
     return ((v & 255u) == kPec ? 1u : 0u) | ((v >> 8) == kPec ? 2u : 0u);
 }
-__device__ __forceinline__ PairPec pairPec(const PairArgs &a, int x, int j, int k, long long node0)
+// Faces of the pair at (x, j, k) behind which a PEC node lies, two bits per face
+// (one per node of the pair): -x +x -y +y -z +z. A neighbour outside the grid
+// counts as none (the wall comes first, as in the general tile body).
+__device__ __forceinline__ unsigned pairPecFaces(const uint8_t *mat, int nx, int ny, int nz, int px, int x, int j, int k,
+                                                 long long node0)
 {
-    PairPec r;
-    const long long sz = (long long)a.px * a.ny;
-    const unsigned own = pecPair(a.mat + node0);
-    r.xm = (own << 1) & 2u;
-    r.xp = x + 1 < a.nx ? own >> 1 : 0u;
-    if (x > 0 && a.mat[node0 - 1] == kPec) r.xm |= 1u;
-    if (x + 2 < a.nx && a.mat[node0 + 2] == kPec) r.xp |= 2u;
-    r.ym = j > 0 ? pecPair(a.mat + node0 - a.px) : 0u;
-    r.yp = j < a.ny - 1 ? pecPair(a.mat + node0 + a.px) : 0u;
-    r.zm = k > 0 ? pecPair(a.mat + node0 - sz) : 0u;
-    r.zp = k < a.nz - 1 ? pecPair(a.mat + node0 + sz) : 0u;
-    return r;
+    const long long sz = (long long)px * ny;
+    const unsigned own = pecPair(mat + node0);
+    unsigned xm = (own << 1) & 2u, xp = x + 1 < nx ? own >> 1 : 0u;
+    if (x > 0 && mat[node0 - 1] == kPec) xm |= 1u;
+    if (x + 2 < nx && mat[node0 + 2] == kPec) xp |= 2u;
+    unsigned f = xm | xp << 2;
+    if (j > 0) f |= pecPair(mat + node0 - px) << 4;
+    if (j < ny - 1) f |= pecPair(mat + node0 + px) << 6;
+    if (k > 0) f |= pecPair(mat + node0 - sz) << 8;
+    if (k < nz - 1) f |= pecPair(mat + node0 + sz) << 10;
+    return f;
 }
 __device__ __forceinline__ void negWhere(float2 &v, unsigned mask, float2 own)
 {
@@ -332,7 +337,6 @@ template <class L, bool DIEL>
 __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(const __grid_constant__ PairArgs a)
 {
     extern __shared__ __align__(128) float sm[];
-    __shared__ double red[L::kThreads / 32];
     __shared__ __align__(8) unsigned long long full[L::kStages];
     const PairShape &g = a.sh;
     const int tid = threadIdx.x;
@@ -421,13 +425,13 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
         else
             scatterAir2(inc, out, negZero);
     };
-    const unsigned energyBits = (a.epart[0] ? kPairEnergy0 : 0u) | (a.epart[1] ? kPairEnergy1 : 0u);
+    const unsigned energyBits = (a.epair[0] ? kPairEnergy0 : 0u) | (a.epair[1] ? kPairEnergy1 : 0u);
     auto flagsAt = [&](int k) -> unsigned { return k <= kB ? colFlags[k] | energyBits : 0u; };
-    // material ids of the pair (none where the plane's flags say neither PEC
-    // nor dielectric), fetched two planes ahead, the flags three
-    auto idsAt = [&](int k, unsigned f) -> unsigned {
-        if (!(f & (kPairPec | kPairDiel)) || !valid) return 0u;
-        return *reinterpret_cast<const unsigned short *>(a.mat + k * sz + colOff);
+    // material word of the pair (only its dead nodes where the plane's flags say
+    // neither PEC nor dielectric), fetched two planes ahead, the flags three
+    auto wordAt = [&](int k, unsigned f) -> unsigned {
+        if (!(f & (kPairPec | kPairDiel)) || !valid) return dead << 18;
+        return a.words[(k * sz + colOff) >> 1];
     };
     auto loadStub = [&](unsigned m, int k, float2(&v)[3]) {
 #pragma unroll
@@ -453,9 +457,8 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
         for (int t = 0; t < 3; ++t) vs[b][t] = make_float2(0.f, 0.f);
     }
     unsigned f0 = flagsAt(kA), f1 = flagsAt(kA + 1), f2 = flagsAt(kA + 2), fPrev = 0;
-    unsigned m0 = matWord(idsAt(kA, f0), dead), m1 = matWord(idsAt(kA + 1, f1), dead), mPrev = 0;
+    unsigned m0 = wordAt(kA, f0), m1 = wordAt(kA + 1, f1), mPrev = 0;
     if constexpr (DIEL) loadStub(m0, kA, vs[0]);
-    double en0 = 0.0, en1 = 0.0;
     bool waitOk = true;
     int si = 0;
     unsigned phase = 0;
@@ -487,21 +490,24 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
             }
             if (fPrev & kPairPec)
             {
-                const PairPec q = pairPec(a, x, j, kk, kk * sz + colOff);
-#pragma unroll
-                for (int t = 0; t < 2; ++t)
+                const unsigned q = mPrev >> 20;
+                if (q)
                 {
-                    if (q.xm) negWhere(inc[t], q.xm, ld2(ex + e0 + t * L::exSlot));
-                    if (q.xp) negWhere(inc[2 + t], q.xp, ld2(ex + e0 + (2 + t) * L::exSlot));
-                    if (q.ym) negWhere(inc[4 + t], q.ym, ld2(ex + e0 + (4 + t) * L::exSlot));
-                    if (q.yp) negWhere(inc[6 + t], q.yp, ld2(ex + e0 + (6 + t) * L::exSlot));
-                    negWhere(inc[8 + t], q.zm, z89[B ^ 1][t]);
-                    negWhere(inc[10 + t], q.zp, z1011[B ^ 1][t]);
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+                    {
+                        negWhere(inc[t], q & 3u, ld2(ex + e0 + t * L::exSlot));
+                        negWhere(inc[2 + t], (q >> 2) & 3u, ld2(ex + e0 + (2 + t) * L::exSlot));
+                        negWhere(inc[4 + t], (q >> 4) & 3u, ld2(ex + e0 + (4 + t) * L::exSlot));
+                        negWhere(inc[6 + t], (q >> 6) & 3u, ld2(ex + e0 + (6 + t) * L::exSlot));
+                        negWhere(inc[8 + t], (q >> 8) & 3u, z89[B ^ 1][t]);
+                        negWhere(inc[10 + t], (q >> 10) & 3u, z1011[B ^ 1][t]);
+                    }
                 }
             }
             const unsigned live = 3u & ~(mPrev >> 18);
-            if (fPrev & kPairSpec) pairSpec(a, 1, kk * sz + colOff, true, live, inc);
-            if (fPrev & kPairEnergy1) en1 += pairEnergy(inc, live);
+            if (fPrev & kPairSpec) pairSpec(a, 1, (long long)kk * a.ny + j, kk * sz + colOff, true, live, inc);
+            if (fPrev & kPairEnergy1) a.epair[1][(kk * sz + colOff) >> 1] = pairEnergy(inc, live);
         }
         float2 o[12];
         scatter(ownLanes, fPrev, inc, vs[B ^ 1], mPrev, o);
@@ -534,7 +540,7 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
 
     auto plane = [&](auto par, int k) {
         constexpr int B = decltype(par)::value;
-        const unsigned ids2 = idsAt(k + 2, f2), f3 = flagsAt(k + 3);
+        const unsigned m2 = wordAt(k + 2, f2), f3 = flagsAt(k + 3);
         float2 s1011[2], vsNext[3];
         if (k <= kB)
         {
@@ -567,24 +573,24 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
                     if (k == a.nz - 1) inc[10 + t] = mul2(inc[10 + t], splat2(a.rho), negZero);
                 }
                 const long long node0 = k * sz + colOff;
-                if ((f0 & kPairPec) && valid)
+                const unsigned q = m0 >> 20;
+                if (q)
                 {
-                    const PairPec q = pairPec(a, x, j, k, node0);
 #pragma unroll
                     for (int t = 0; t < 2; ++t)
                     {
-                        if (q.xm) negWhere(inc[t], q.xm, ld2(st + t * L::sX + oX));
-                        if (q.xp) negWhere(inc[2 + t], q.xp, ld2(st + (2 + t) * L::sX + oX));
-                        if (q.ym) negWhere(inc[4 + t], q.ym, ld2(st + L::offYH + t * L::sY + oX));
-                        if (q.yp) negWhere(inc[6 + t], q.yp, ld2(st + L::offYL + t * L::sY + oX + L::W2));
-                        if (q.zm) negWhere(inc[8 + t], q.zm, ld2(a.in + (8 + t) * a.P + node0));
-                        if (q.zp) negWhere(inc[10 + t], q.zp, ld2(a.in + (10 + t) * a.P + node0));
+                        negWhere(inc[t], q & 3u, ld2(st + t * L::sX + oX));
+                        negWhere(inc[2 + t], (q >> 2) & 3u, ld2(st + (2 + t) * L::sX + oX));
+                        negWhere(inc[4 + t], (q >> 4) & 3u, ld2(st + L::offYH + t * L::sY + oX));
+                        negWhere(inc[6 + t], (q >> 6) & 3u, ld2(st + L::offYL + t * L::sY + oX + L::W2));
+                        if ((q >> 8) & 3u) negWhere(inc[8 + t], (q >> 8) & 3u, ld2(a.in + (8 + t) * a.P + node0));
+                        if ((q >> 10) & 3u) negWhere(inc[10 + t], (q >> 10) & 3u, ld2(a.in + (10 + t) * a.P + node0));
                     }
                 }
                 const unsigned live = 3u & ~(m0 >> 18);
                 const bool mine = own && k >= kc0 && k < kc1;
-                if ((f0 & kPairSpec) && valid) pairSpec(a, 0, node0, mine, live, inc);
-                if ((f0 & kPairEnergy0) && mine) en0 += pairEnergy(inc, live);
+                if ((f0 & kPairSpec) && valid) pairSpec(a, 0, (long long)k * a.ny + j, node0, mine, live, inc);
+                if ((f0 & kPairEnergy0) && mine) a.epair[0][node0 >> 1] = pairEnergy(inc, live);
             }
             // Pulses of dead nodes need not be zeroed here: their neighbours
             // reflect their own (PEC, walls) and the second step writes zeros.
@@ -621,7 +627,7 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
         if (tid == 0 && waitOk && lastIssued < kB) issue(++lastIssued);
         mPrev = m0;
         m0 = m1;
-        m1 = matWord(ids2, dead);
+        m1 = m2;
         fPrev = f0;
         f0 = f1;
         f1 = f2;
@@ -642,24 +648,12 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
     if (!waitOk && tid == 0)
         for (int k = max(kA, lastIssued - L::kStages + 1); k <= lastIssued; ++k)
             mbarWaitBounded(full0 + 8 * ((k - kA) % L::kStages), (unsigned)((k - kA) / L::kStages) & 1u);
-    // ---- energy partials: one per block, zeros in the rest of the list ----
-#pragma unroll
-    for (int st = 0; st < 2; ++st)
-        if (a.epart[st] != nullptr)
-        {
-            const double tot = blockSumDouble(st == 0 ? en0 : en1, red);
-            if (tid == 0) a.epart[st][blockIdx.x] = tot;
-            for (long long b = (long long)gridDim.x + (long long)blockIdx.x * L::kThreads + tid; b < a.nepart;
-                 b += (long long)gridDim.x * L::kThreads)
-                a.epart[st][b] = 0.0;
-            __syncthreads();
-        }
 }
 
 // Flags of every (column, plane): PEC and dielectric nodes from the padded
 // material map (one block per column and plane; PEC within one node of the
 // grown column, the planes below and above included).
-inline __global__ void __launch_bounds__(128) pairMaterialFlags(const uint8_t *__restrict__ mat, int nx, int ny, int nz, int px,
+static __global__ void __launch_bounds__(128) pairMaterialFlags(const uint8_t *__restrict__ mat, int nx, int ny, int nz, int px,
                                                          PairShape g, unsigned *__restrict__ flags)
 {
     const int k = blockIdx.x % nz, col = blockIdx.x / nz;
@@ -681,8 +675,35 @@ inline __global__ void __launch_bounds__(128) pairMaterialFlags(const uint8_t *_
     if ((threadIdx.x & 31) == 0 && f) atomicOr(flags + (long long)col * nz + k, f);
 }
 
+// The material word of every pair, and the first source or monitor entry of
+// every row of nodes (entries are sorted by node).
+static __global__ void __launch_bounds__(256) pairWordKernel(const uint8_t *__restrict__ mat, int nx, int ny, int nz, int px,
+                                                             FastDiv divH, FastDiv divY, unsigned npairs,
+                                                             unsigned *__restrict__ words)
+{
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= npairs) return;
+    const unsigned row = fastDiv(q, divH), k = fastDiv(row, divY);
+    const int x = 2 * (int)(q - row * (unsigned)(px / 2)), j = (int)(row - k * (unsigned)ny);
+    words[q] = matWord(*reinterpret_cast<const unsigned short *>(mat + 2LL * q), x + 1 < nx ? 0u : x < nx ? 2u : 3u) |
+               pairPecFaces(mat, nx, ny, nz, px, x, j, (int)k, 2LL * q) << 20;
+}
+static __global__ void __launch_bounds__(256) pairSpecRows(const SpecEntry *__restrict__ spec, int n, int rows, int px,
+                                                           int *__restrict__ first)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r > rows) return;
+    int lo = 0, hi = n;
+    while (lo < hi)
+    {
+        const int mid = (lo + hi) >> 1;
+        if (spec[mid].node < (long long)r * px) lo = mid + 1; else hi = mid;
+    }
+    first[r] = lo;
+}
+
 // ... and the columns whose grown area holds a source or monitor node.
-inline __global__ void __launch_bounds__(128) pairSpecFlags(const SpecEntry *__restrict__ spec, int n, int ny, int nz, int px,
+static __global__ void __launch_bounds__(128) pairSpecFlags(const SpecEntry *__restrict__ spec, int n, int ny, int nz, int px,
                                                      PairShape g, unsigned *__restrict__ flags)
 {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -693,6 +714,17 @@ inline __global__ void __launch_bounds__(128) pairSpecFlags(const SpecEntry *__r
         for (int tx = max(x / g.TX - 1, 0); tx <= min(x / g.TX + 1, g.ntx - 1); ++tx)
             if (x >= tx * g.TX - 2 && x < tx * g.TX + g.TX + 2 && j >= ty * g.TY - 1 && j <= ty * g.TY + g.TY)
                 atomicOr(flags + (long long)(ty * g.ntx + tx) * nz + k, (unsigned)kPairSpec);
+}
+
+// The tiles' energy sums from the pairs' shares: block (tile, energy step), in
+// the order of blockSumDouble as the single-step kernels use it.
+static __global__ void __launch_bounds__(kBlock) pairEnergySums(const double *__restrict__ epair, long long npairs,
+                                                         double *__restrict__ epart, int nblocks)
+{
+    __shared__ double red[kBlock / 32];
+    const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
+    const double tot = blockSumDouble(q < npairs ? epair[blockIdx.y * npairs + q] : 0.0, red);
+    if (threadIdx.x == 0) epart[(long long)blockIdx.y * nblocks + blockIdx.x] = tot;
 }
 
 } // namespace tlmk

@@ -26,7 +26,7 @@
 //
 // The arithmetic of a node is that of the interior and general tile bodies in
 // their order: pulses, stubs and samples are bitwise the same. Energy steps
-// leave every pair's FP64 share in `epair`; residentEnergy adds those up in the
+// leave every pair's FP64 share in `epair`; pairEnergySums adds those up in the
 // order of the single-step kernels' tiles, so the energies are the same too.
 #pragma once
 
@@ -177,15 +177,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentKernel(const __gr
             const int o = 2 * q;
             at[m] = o;
             unsigned f = kResUsed;
-            const unsigned own = pecPair(a.mat + n0);
-            unsigned xm = (own << 1) & 2u, xp = x + 1 < a.nx ? own >> 1 : 0u;
-            if (x > 0 && a.mat[n0 - 1] == kPec) xm |= 1u;
-            if (x + 2 < a.nx && a.mat[n0 + 2] == kPec) xp |= 2u;
-            f |= xm | (xp << 2);
-            if (j > 0) f |= pecPair(a.mat + n0 - a.px) << 4;
-            if (j < a.ny - 1) f |= pecPair(a.mat + n0 + a.px) << 6;
-            if (k > 0) f |= pecPair(a.mat + n0 - sz) << 8;
-            if (k < a.nz - 1) f |= pecPair(a.mat + n0 + sz) << 10;
+            f |= pairPecFaces(a.mat, a.nx, a.ny, a.nz, a.px, x, j, k, n0);
             if (x == 0) f |= kResWallXlo;
             if (x == a.nx - 1) f |= kResWallX0;
             if (x + 1 == a.nx - 1) f |= kResWallX1;
@@ -455,17 +447,6 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentKernel(const __gr
                         *reinterpret_cast<float2 *>(a.stub + t * a.P + node[m]) = ld2(stubs + t * L::SS + at[m]);
                 }
         }
-}
-
-// The tiles' energy sums from the pairs' shares: block (tile, energy step), in
-// the order of blockSumDouble as the single-step kernels use it.
-__global__ void __launch_bounds__(kBlock) residentEnergy(const double *__restrict__ epair, long long npairs,
-                                                         double *__restrict__ epart, int nblocks)
-{
-    __shared__ double red[kBlock / 32];
-    const long long q = (long long)blockIdx.x * kBlock + threadIdx.x;
-    const double tot = blockSumDouble(q < npairs ? epair[blockIdx.y * npairs + q] : 0.0, red);
-    if (threadIdx.x == 0) epart[(long long)blockIdx.y * nblocks + blockIdx.x] = tot;
 }
 
 } // namespace tlmk

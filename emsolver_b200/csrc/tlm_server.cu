@@ -131,9 +131,10 @@ size_t footprintOf(const tlm_grid &g, const std::vector<uint8_t> &mat, const tlm
             break;
         }
     const size_t steps = (size_t)std::max(cfg.total_steps, 1);
-    // (large FP32 grids step two steps per pass, with a second set of stubs)
-    const size_t stubSets = tlmi::pairStorage(cfg.storage, (long long)P) ? 2 : 1;
-    return 2 * 12 * P * sb + (diel ? stubSets * 3 * P * rb : 0) + P + steps * (nports * 2 + nprobes * 3 + 1) * 8 +
+    // (large FP32 grids step two steps per pass, with a second set of stubs and
+    // every node pair's energy share and material word)
+    const bool pair = tlmi::pairStorage(cfg.storage, (long long)P);
+    return 2 * 12 * P * sb + (diel ? (pair ? 2 : 1) * 3 * P * rb : 0) + (pair ? 6 * P : 0) + P + steps * (nports * 2 + nprobes * 3 + 1) * 8 +
            nports * nfreq * 32 + steps * rb + (1u << 20);
 }
 

@@ -71,6 +71,8 @@ void freeMonitors(tlm_solver *h)
     h->pair.reset();
     h->pairTried = false;
     devFree(h, h->dPairFlags);
+    devFree(h, h->dPairWord);
+    devFree(h, h->dSpecRow);
     devFree(h, h->dStubAlt);
     h->resTried = false;
     h->resBy = 0;
@@ -649,6 +651,17 @@ tlm_status timeLaunch(tlm_solver *h, int steps, cudaEvent_t *after)
     return TLM_OK;
 }
 
+// Whether a single step runs its interior tiles in the staged kernel. FP32
+// grids below 2^20 nodes do not: there the fork and join of two kernels costs
+// more than staging gains (80x84x77 dipole 16.8 us staged, 12.6 us in one
+// kernel; 100^3 heterogeneous 26.2 and 23.8 us). A stage wait limit in the
+// configuration asks for the staged kernel.
+bool stagedStep(const tlm_solver *h)
+{
+    return h->nStaged > 0 && !h->stateIncident &&
+           (h->storage != TLM_STORE_F32 || h->P >= kPairMinNodes || h->cfg.stage_wait_us != 0);
+}
+
 template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long eFirst)
 {
     const tlmk::StepArgs<S> a = stepArgs<S>(h, n, i, eFirst);
@@ -657,7 +670,7 @@ template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long 
     if (surfaceActive(h)) TLM_TRY(launchSurface(h, n));  // reads the same input buffer, first
     if constexpr (std::is_same<S, float>::value)
     {
-        if (h->nStaged > 0 && !h->stateIncident)
+        if (stagedStep(h))
         {
             // the listed tiles run beside the staged ones (disjoint outputs,
             // the same input), on the side stream between a fork and a join
@@ -683,7 +696,7 @@ template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long 
     }
     else if constexpr (std::is_same<S, __half>::value || std::is_same<S, __nv_bfloat16>::value)
     {
-        if (h->nStaged > 0 && !h->stateIncident)
+        if (stagedStep(h))
         {
             // as FP32: the listed tiles beside the staged ones
             if (h->nListed > 0)
@@ -789,9 +802,8 @@ tlm_status ensurePair(tlm_solver *h)
     h->pairTried = true;
     TensorMapEncoder encode = tensorMapEncoder();
     if (!encode) return TLM_OK;
-    if (h->dStub)
     {
-        const size_t need = 3 * (size_t)h->P * sizeof(float);
+        const size_t need = (h->dStub ? 3 : 0) * (size_t)h->P * sizeof(float) + (size_t)(h->P / 2) * 12;
         if (!poolCovers(h->device, need) && poolAvailable(h->device) < need + ((size_t)256 << 20)) return TLM_OK;
     }
     int sms = 0;
@@ -799,9 +811,8 @@ tlm_status ensurePair(tlm_solver *h)
     auto plan = std::make_shared<PairPlan>();
     choosePairShape(h->ny, h->nz, h->px, sms, plan->sh, plan->layout);
     const tlmk::PairShape &g = plan->sh;
-    // the kernel's lane offsets within a plane are 32-bit byte offsets, and
-    // its energy partials take the single-step kernels' places
-    if ((long long)h->px * h->ny > (1LL << 28) || (long long)g.ntx * g.nty * g.nchunk > h->nblocks) return TLM_OK;
+    // the kernel's lane offsets within a plane are 32-bit byte offsets
+    if ((long long)h->px * h->ny > (1LL << 28)) return TLM_OK;
     tlm_status st = TLM_OK;
     bool ok = true;
     withPairLayout(plan->layout, [&](auto L) {
@@ -830,6 +841,7 @@ tlm_status ensurePair(tlm_solver *h)
     });
     TLM_TRY(st);
     if (!ok) return TLM_OK;
+    if (!h->dEpair && devAlloc(h, &h->dEpair, (size_t)(h->P / 2) * sizeof(double)) != TLM_OK) return TLM_OK;
     if (h->dStub)
     {
         if (devAlloc(h, &h->dStubAlt, 3 * (size_t)h->P * sizeof(float)) != TLM_OK) return TLM_OK;
@@ -839,6 +851,15 @@ tlm_status ensurePair(tlm_solver *h)
     TLM_TRY(devAlloc(h, &h->dPairFlags, nf * sizeof(unsigned)));
     TLM_CU(h, cudaMemsetAsync(h->dPairFlags, 0, nf * sizeof(unsigned), h->stream));
     tlmk::pairMaterialFlags<<<(unsigned)nf, 128, 0, h->stream>>>(h->dMat, h->nx, h->ny, h->nz, h->px, g, h->dPairFlags);
+    const long long npairs = h->P / 2, rows = (long long)h->ny * h->nz;
+    if (devAlloc(h, &h->dPairWord, (size_t)npairs * sizeof(unsigned)) != TLM_OK ||
+        devAlloc(h, &h->dSpecRow, (size_t)(rows + 1) * sizeof(int)) != TLM_OK)
+        return TLM_OK;
+    tlmk::pairWordKernel<<<(unsigned)((npairs + 255) / 256), 256, 0, h->stream>>>(
+        h->dMat, h->nx, h->ny, h->nz, h->px, tlmk::makeFastDiv((unsigned)(h->px / 2)),
+        tlmk::makeFastDiv((unsigned)h->ny), (unsigned)npairs, h->dPairWord);
+    tlmk::pairSpecRows<<<(unsigned)((rows + 256) / 256), 256, 0, h->stream>>>(h->dSpec, h->specCount, (int)rows, h->px,
+                                                                            h->dSpecRow);
     if (h->specCount)
         tlmk::pairSpecFlags<<<(h->specCount + 127) / 128, 128, 0, h->stream>>>(h->dSpec, h->specCount, h->ny, h->nz,
                                                                                h->px, g, h->dPairFlags);
@@ -870,7 +891,6 @@ tlm_status launchPair(tlm_solver *h, int n, int i, long long eFirst)
     a.out = s0.out;
     a.stubIn = static_cast<const float *>(h->dStub);
     a.stubOut = static_cast<float *>(h->dStubAlt);
-    a.mat = s0.mat;
     a.yhat = s0.yhat;
     a.ghat = s0.ghat;
     a.ntable = (int)h->epsr.size();
@@ -881,15 +901,15 @@ tlm_status launchPair(tlm_solver *h, int n, int i, long long eFirst)
     a.nz = h->nz;
     a.px = h->px;
     a.rho = s0.rho;
+    a.words = h->dPairWord;
     a.spec = h->dSpec;
-    a.nspec = h->specCount;
+    a.specRow = h->dSpecRow;
     a.sv[0] = s0.sv;
     a.sv[1] = s1.sv;
     a.samples[0] = s0.samples;
     a.samples[1] = s1.samples;
-    a.epart[0] = s0.epart;
-    a.epart[1] = s1.epart;
-    a.nepart = h->nblocks;
+    a.epair[0] = s0.epart ? h->dEpair : nullptr;
+    a.epair[1] = s1.epart ? h->dEpair : nullptr;  // (at most one of two steps is an energy step)
     a.neg_zero = -0.0f;
     a.stage_wait_ns = s0.stage_wait_ns;
     a.fault = h->dFault;
@@ -903,6 +923,8 @@ tlm_status launchPair(tlm_solver *h, int n, int i, long long eFirst)
         else
             tlmk::stepPairKernel<Layout, false><<<blocks, Layout::kThreads, Layout::smemBytes, h->stream>>>(a);
     });
+    if (double *epart = s0.epart ? s0.epart : s1.epart)
+        tlmk::pairEnergySums<<<(unsigned)h->nblocks, kBlock, 0, h->stream>>>(h->dEpair, h->P / 2, epart, h->nblocks);
     TLM_CU(h, cudaGetLastError());
     if (after) TLM_CU(h, cudaEventRecord(after, h->stream));
     if (h->dStubAlt) std::swap(h->dStub, h->dStubAlt);
@@ -1052,7 +1074,7 @@ tlm_status launchResident(tlm_solver *h, int n, int i, int steps, long long eFir
     if (e0 < (long long)n + steps)
     {
         const int ne = (int)(((long long)n + steps - 1 - e0) / 16 + 1);
-        tlmk::residentEnergy<<<dim3((unsigned)h->nblocks, (unsigned)ne), kBlock, 0, h->stream>>>(
+        tlmk::pairEnergySums<<<dim3((unsigned)h->nblocks, (unsigned)ne), kBlock, 0, h->stream>>>(
             h->dEpair, h->P / 2, h->dEpart + (size_t)((e0 - eFirst) / 16) * h->nblocks, h->nblocks);
         TLM_CU(h, cudaGetLastError());
     }
@@ -2594,7 +2616,7 @@ tlm_status tlm_step_launches(tlm_handle h, int *per_step)
     TLM_TRY(checkHandle(h));
     if (!per_step) return h->fail(TLM_EINVAL, "null output");
     TLM_TRY(prepare(h));
-    *per_step = (h->nStaged > 0 ? (h->nListed > 0 ? 2 : 1) : 1) + (surfaceActive(h) ? 1 : 0);
+    *per_step = (stagedStep(h) ? (h->nListed > 0 ? 2 : 1) : 1) + (surfaceActive(h) ? 1 : 0);
     return TLM_OK;
 }
 

@@ -4,8 +4,9 @@ The pass computes the same node updates in the same order as two single
 steps, so pulses, stubs, probe and port records are compared bit for bit: with
 the single-step kernel (tlm_config.no_staging = 1) on grids whose sizes cut the
 columns and plane ranges raggedly, and with the oracle. The energy is an FP64
-sum of squares in another order: partial sums of at most a few thousand terms
-each, so relative 1e-12."""
+sum of squares, on the device in the order of the single-step tiles, in the
+oracle in another: partial sums of at most a few thousand terms each, so
+relative 1e-12."""
 import numpy as np
 import pytest
 

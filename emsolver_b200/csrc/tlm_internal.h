@@ -236,6 +236,7 @@ struct tlm_solver
     bool prepared = false;
     int nsamp = 0;
     int specCount = 0;     // entries of dSpec
+    long long injLo = 0, injHi = -1;  // first and last padded node with a source
 
     // time-loop state
     int curStep = 0;       // steps enqueued

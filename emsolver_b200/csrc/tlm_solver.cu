@@ -432,6 +432,14 @@ tlm_status prepare(tlm_solver *h)
         ents.push_back({ monNodes[sidx], tlmk::kSample, sidx, 0.0f, 0 });
     std::stable_sort(ents.begin(), ents.end(),
                      [](const SpecEntry &a, const SpecEntry &b) { return a.node < b.node; });
+    h->injLo = 0;
+    h->injHi = -1;
+    for (const SpecEntry &se : ents)
+        if (se.kind == tlmk::kInject)
+        {
+            if (h->injHi < h->injLo) h->injLo = se.node;
+            h->injHi = se.node;
+        }
     std::vector<int> tile(h->nblocks + 1, 0);
     {
         size_t e = 0;

@@ -18,8 +18,8 @@
 // one thread and is updated in step order in the storage's real type, so
 // FP32 results are bitwise the reference's.
 //
-// The far field (ComputeFarFieldFromHuygens, TlmSolver.cpp:805-916) is one
-// block per direction summing the faces' radiation vectors in FP64.
+// The far field (ComputeFarFieldFromHuygens, TlmSolver.cpp:805-916) is summed on
+// the device in FP64, a few directions per block.
 #include "tlm_b200.h"
 #include "tlm_internal.h"
 
@@ -35,6 +35,8 @@ using namespace tlmi;
 
 namespace tlmk {
 
+constexpr int kSurfaceThreads = 128;
+
 template <class S> struct SurfaceArgs
 {
     using R = typename Traits<S>::R;
@@ -46,6 +48,7 @@ template <class S> struct SurfaceArgs
     R rho, scale;
     const SpecEntry *spec;  // node-sorted sources and samples
     int nspec;
+    long long injLo, injHi; // first and last node with a source (injLo > injHi: none)
     R sv;                   // source value of step n
     // PEC-surface faces
     const long long *jsNode;  // face code: padded node * 8 + axis * 2 + (normal sign < 0)
@@ -74,25 +77,33 @@ __device__ void incidentAt(const SurfaceArgs<S> &a, long long node, int i, int j
     const long long stride[3] = { 1, a.px, (long long)a.px * a.ny };
     const int co[3] = { i, j, k };
     const int dims[3] = { a.nx, a.ny, a.nz };
+    // loads first, all independent: the pulse that arrives on each slot (the
+    // node's own one from an outer wall) and the neighbours' materials
+    uint8_t mat[6];
 #pragma unroll
     for (int s = 0; s < 12; ++s)
     {
-        const R own = loadOne<S>(a.in, s * a.P + node, a.scale);
-        if (a.incident)
-        {
-            inc[s] = own;
-            continue;
-        }
         const int ax = s >> 2, side = (s >> 1) & 1;
         const int q = co[ax] + (side ? 1 : -1);
-        if (q < 0 || q >= dims[ax])
-            inc[s] = a.rho * own;
-        else
+        const bool in = !a.incident && q >= 0 && q < dims[ax];
+        const long long nb = in ? node + (side ? stride[ax] : -stride[ax]) : node;
+        inc[s] = loadOne<S>(a.in, (in ? s ^ 2 : s) * a.P + nb, a.scale);
+        if (!(s & 1)) mat[s >> 1] = in ? a.mat[nb] : 0;
+    }
+    if (!a.incident)
+    {
+#pragma unroll
+        for (int s = 0; s < 12; ++s)
         {
-            const long long nb = node + (side ? stride[ax] : -stride[ax]);
-            inc[s] = (a.mat[nb] == kPec) ? -own : loadOne<S>(a.in, (s ^ 2) * a.P + nb, a.scale);
+            const int ax = s >> 2, side = (s >> 1) & 1;
+            const int q = co[ax] + (side ? 1 : -1);
+            if (q < 0 || q >= dims[ax])
+                inc[s] = a.rho * inc[s];
+            else if (mat[s >> 1] == kPec)
+                inc[s] = -loadOne<S>(a.in, s * a.P + node, a.scale);
         }
     }
+    if (node < a.injLo || node > a.injHi) return;
     // soft sources of this node, in the order the step kernel applies them
     int lo = 0, hi = a.nspec;
     while (lo < hi)
@@ -111,15 +122,48 @@ __device__ void incidentAt(const SurfaceArgs<S> &a, long long node, int i, int j
     }
 }
 
+// (a face node below 2^32 takes 32-bit divisions; every grid of 16-bit pulses
+// or wider that fits the card is below)
 __device__ __forceinline__ void cellOfNode(long long node, int px, int ny, int *i, int *j, int *k)
 {
-    const long long r = node / px;
-    *i = (int)(node - r * px);
-    *j = (int)(r % ny);
-    *k = (int)(r / ny);
+    if (node >> 32)
+    {
+        const long long r = node / px;
+        *i = (int)(node - r * px);
+        *j = (int)(r % ny);
+        *k = (int)(r / ny);
+        return;
+    }
+    const unsigned n = (unsigned)node, r = n / (unsigned)px;
+    *i = (int)(n - r * (unsigned)px);
+    *j = (int)(r % (unsigned)ny);
+    *k = (int)(r / (unsigned)ny);
 }
 
-template <class S> __global__ void __launch_bounds__(256) surfaceMonitorKernel(const SurfaceArgs<S> a)
+// N accumulators of a face, 16-byte loads and stores (N * sizeof(R) is a
+// multiple of 16, and so is every face's offset).
+template <class R, int N> __device__ __forceinline__ void loadAcc(const R *p, R (&v)[N])
+{
+#pragma unroll
+    for (int q = 0; q < N * (int)sizeof(R) / 16; ++q)
+        reinterpret_cast<int4 *>(v)[q] = reinterpret_cast<const int4 *>(p)[q];
+}
+template <class R, int N> __device__ __forceinline__ void storeAcc(R *p, const R (&v)[N])
+{
+#pragma unroll
+    for (int q = 0; q < N * (int)sizeof(R) / 16; ++q)
+        reinterpret_cast<int4 *>(p)[q] = reinterpret_cast<const int4 *>(v)[q];
+}
+
+// One thread per face or cut-plane point. Bound by the chain of dependent
+// loads (a face touches 12 pulses, 6 materials and its accumulators, scattered
+// for x faces, and the faces of a 96^3 Huygens box fill a third of the
+// card's threads), so the chain is kept at two: the face's code and
+// accumulators, then everything else; only a PEC neighbour and a face among the
+// sources add one.
+// On a B200, 48,600 Huygens faces of a 96^3 grid, FP32, caches cold: 20.0 ->
+// 8.5 us per step.
+template <class S> __global__ void __launch_bounds__(kSurfaceThreads) surfaceMonitorKernel(const SurfaceArgs<S> a)
 {
     using R = typename Traits<S>::R;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -130,6 +174,8 @@ template <class S> __global__ void __launch_bounds__(256) surfaceMonitorKernel(c
     {
         // TlmSolver.cpp:632-646
         const long long code = a.jsNode[t];
+        alignas(16) R acc[4];
+        if (a.doDft) loadAcc<R, 4>(a.jsAcc + t * 4, acc);
         const long long node = code >> 3;
         const int ax = (int)((code >> 1) & 3);
         int i, j, k;
@@ -139,11 +185,11 @@ template <class S> __global__ void __launch_bounds__(256) surfaceMonitorKernel(c
         a.jsInst[t] = sqrt(h1 * h1 + h2 * h2);
         if (a.doDft)
         {
-            R *acc = a.jsAcc + t * 4;
             acc[0] = acc[0] + h1 * a.cph;
             acc[1] = acc[1] - h1 * a.sph;
             acc[2] = acc[2] + h2 * a.cph;
             acc[3] = acc[3] - h2 * a.sph;
+            storeAcc<R, 4>(a.jsAcc + t * 4, acc);
         }
         return;
     }
@@ -152,6 +198,8 @@ template <class S> __global__ void __launch_bounds__(256) surfaceMonitorKernel(c
     {
         // TlmSolver.cpp:660-671: E_t ~ -V_t, eta0 H_t ~ -ZI_t
         const long long code = a.huyNode[u];
+        alignas(16) R acc[8];
+        loadAcc<R, 8>(a.huyAcc + u * 8, acc);
         const long long node = code >> 3;
         const int ax = (int)((code >> 1) & 3);
         int i, j, k;
@@ -160,7 +208,6 @@ template <class S> __global__ void __launch_bounds__(256) surfaceMonitorKernel(c
         const int t1 = ax == 0 ? 1 : 0, t2 = ax == 2 ? 1 : 2;
         const R e1 = -nodeVoltage(inc, t1), e2 = -nodeVoltage(inc, t2);
         const R m1 = -circulation(inc, t1), m2 = -circulation(inc, t2);
-        R *acc = a.huyAcc + u * 8;
         acc[0] = acc[0] + e1 * a.cph;
         acc[1] = acc[1] - e1 * a.sph;
         acc[2] = acc[2] + e2 * a.cph;
@@ -169,6 +216,7 @@ template <class S> __global__ void __launch_bounds__(256) surfaceMonitorKernel(c
         acc[5] = acc[5] - m1 * a.sph;
         acc[6] = acc[6] + m2 * a.cph;
         acc[7] = acc[7] - m2 * a.sph;
+        storeAcc<R, 8>(a.huyAcc + u * 8, acc);
         return;
     }
     u -= nh;
@@ -200,80 +248,170 @@ template <class S> __global__ void __launch_bounds__(256) surfaceMonitorKernel(c
     }
 }
 
-// Far field: block d = direction (theta index d / nPhi, phi index d % nPhi).
-// Per face the equivalent currents J' = n x (eta0 H), M = -(n x E) in world
-// components (TlmSolver.cpp:829-848), projected on theta/phi and summed with
-// e^{+j k0 r.pos} into N and L (TlmSolver.cpp:860-890); sums in FP64 with a
-// fixed-order block reduction. U = |L_phi + N_theta|^2 + |L_theta - N_phi|^2.
-template <class R>
-__global__ void __launch_bounds__(256)
-    farFieldKernel(const R *__restrict__ acc, const long long *__restrict__ code, const float *__restrict__ pos,
-                   int nh, R k0, int nTheta, int nPhi, R *__restrict__ U)
+// Far field: a block takes kFarDirs directions (theta index d / nPhi, phi index
+// d % nPhi) and one of gridDim.y slices of the faces. Per face the equivalent
+// currents are J' = n x (eta0 H), M = -(n x E) (TlmSolver.cpp:829-848); summed
+// with e^{+j k0 r.pos} they give N and L (TlmSolver.cpp:860-890), here as world
+// components, FP64 throughout, and projected on theta and phi after the sum:
+// U = |L_phi + N_theta|^2 + |L_theta - N_phi|^2. A face has only two components
+// of each, so that costs the same 16 fused multiply-adds as summing projections,
+// and a face is read, signed and widened once for all the block's directions.
+// Sums run in a fixed order: a thread's faces, lanes, warps, slices. With more
+// than one slice the blocks leave their sums in `part` for farFieldFinish.
+// Bound by issue (sine, cosine and 16 FP64 operations per face and direction).
+// 37 x 73 directions of 48,600 FP32 faces on a B200: 1584 -> 421 us (one block of
+// 256 threads per direction, its projections summed, before).
+constexpr int kFarDirs = 4, kFarThreads = 128;
+
+template <class R> __device__ __forceinline__ void sinCos(R x, R *s, R *c)
 {
-    __shared__ double red[8][8];
-    const int d = blockIdx.x;
-    const int ti = d / nPhi, pj = d % nPhi;
+    if constexpr (std::is_same<R, float>::value)
+        sincosf(x, s, c);
+    else
+        sincos(x, s, c);
+}
+
+// Unit vectors of direction d: r, theta and (x and y of) phi.
+template <class R>
+__device__ __forceinline__ void farDirection(int d, int nTheta, int nPhi, R (&rh)[3], R (&tv)[3], R (&pv)[2])
+{
     const R pi = R(3.14159265358979323846);
-    const R th = pi * R(ti) / R(nTheta - 1);
-    const R ph = R(2) * pi * R(pj) / R(nPhi - 1);
+    const R th = pi * R(d / nPhi) / R(nTheta - 1);
+    const R ph = R(2) * pi * R(d % nPhi) / R(nPhi - 1);
     const R st = sin(th), ct = cos(th), cp = cos(ph), sp = sin(ph);
-    const R rh[3] = { st * cp, st * sp, ct };
-    const R tv[3] = { ct * cp, ct * sp, -st };
-    const R pv[2] = { -sp, cp };
-    double s[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };  // Nt, Np, Lt, Lp (re, im)
-    for (int f = threadIdx.x; f < nh; f += blockDim.x)
+    rh[0] = st * cp, rh[1] = st * sp, rh[2] = ct;
+    tv[0] = ct * cp, tv[1] = ct * sp, tv[2] = -st;
+    pv[0] = -sp, pv[1] = cp;
+}
+
+// U of direction d from its sums: N (re, im per component), then L.
+template <class R>
+__device__ __forceinline__ R farIntensity(const double (&v)[12], int d, int nTheta, int nPhi)
+{
+    R rh[3], tv[3], pv[2];
+    farDirection(d, nTheta, nPhi, rh, tv, pv);
+    double t[2][2], p[2][2];  // [N, L][re, im]
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+        {
+            const double x = v[q * 6 + c], y = v[q * 6 + 2 + c], z = v[q * 6 + 4 + c];
+            t[q][c] = x * (double)tv[0] + y * (double)tv[1] + z * (double)tv[2];
+            p[q][c] = x * (double)pv[0] + y * (double)pv[1];
+        }
+    const double aR = p[1][0] + t[0][0], aI = p[1][1] + t[0][1];
+    const double bR = t[1][0] - p[0][0], bI = t[1][1] - p[0][1];
+    return (R)(aR * aR + aI * aI + bR * bR + bI * bI);
+}
+
+template <class R>
+__global__ void __launch_bounds__(kFarThreads, 3)
+    farFieldKernel(const R *__restrict__ acc, const long long *__restrict__ code, const float *__restrict__ pos,
+                   int nh, R k0, int nTheta, int nPhi, R *__restrict__ U, double *__restrict__ part)
+{
+    __shared__ double red[kFarThreads / 32][kFarDirs * 12];
+    const int nd = nTheta * nPhi, d0 = blockIdx.x * kFarDirs;
+    R rh[kFarDirs][3];
+#pragma unroll
+    for (int q = 0; q < kFarDirs; ++q)
     {
-        const R *a = acc + (long long)f * 8;
-        const int ax = (int)((code[f] >> 1) & 3);
-        const int t1 = ax == 0 ? 1 : 0, t2 = ax == 2 ? 1 : 2;
-        const R sa = ax == 1 ? R(-1) : R(1);
-        const R sg = (code[f] & 1) ? R(-1) : R(1);  // outward normal sign
-        R jR[3] = { 0, 0, 0 }, jI[3] = { 0, 0, 0 }, mR[3] = { 0, 0, 0 }, mI[3] = { 0, 0, 0 };
-        jR[t2] = sg * sa * a[4];
-        jI[t2] = sg * sa * a[5];
-        jR[t1] = -sg * sa * a[6];
-        jI[t1] = -sg * sa * a[7];
-        mR[t2] = -sg * sa * a[0];
-        mI[t2] = -sg * sa * a[1];
-        mR[t1] = sg * sa * a[2];
-        mI[t1] = sg * sa * a[3];
-        const R px = R(pos[3 * f]), py = R(pos[3 * f + 1]), pz = R(pos[3 * f + 2]);
-        const R pha = k0 * (rh[0] * px + rh[1] * py + rh[2] * pz);
-        const double c = (double)cos(pha), sn = (double)sin(pha);
-        const double jt[2] = { (double)(jR[0] * tv[0] + jR[1] * tv[1] + jR[2] * tv[2]),
-                               (double)(jI[0] * tv[0] + jI[1] * tv[1] + jI[2] * tv[2]) };
-        const double jp[2] = { (double)(jR[0] * pv[0] + jR[1] * pv[1]), (double)(jI[0] * pv[0] + jI[1] * pv[1]) };
-        const double mt[2] = { (double)(mR[0] * tv[0] + mR[1] * tv[1] + mR[2] * tv[2]),
-                               (double)(mI[0] * tv[0] + mI[1] * tv[1] + mI[2] * tv[2]) };
-        const double mp[2] = { (double)(mR[0] * pv[0] + mR[1] * pv[1]), (double)(mI[0] * pv[0] + mI[1] * pv[1]) };
-        s[0] += jt[0] * c - jt[1] * sn;
-        s[1] += jt[0] * sn + jt[1] * c;
-        s[2] += jp[0] * c - jp[1] * sn;
-        s[3] += jp[0] * sn + jp[1] * c;
-        s[4] += mt[0] * c - mt[1] * sn;
-        s[5] += mt[0] * sn + mt[1] * c;
-        s[6] += mp[0] * c - mp[1] * sn;
-        s[7] += mp[0] * sn + mp[1] * c;
+        R tv[3], pv[2];
+        farDirection(min(d0 + q, nd - 1), nTheta, nPhi, rh[q], tv, pv);
     }
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-        for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], o);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0)
+    double s[kFarDirs][12] = {};
+    const int f0 = (int)((long long)nh * blockIdx.y / gridDim.y), f1 = (int)((long long)nh * (blockIdx.y + 1) / gridDim.y);
+    for (int f = f0 + (int)threadIdx.x; f < f1; f += kFarThreads)
     {
+        alignas(16) R a[8];
+        loadAcc<R, 8>(acc + (long long)f * 8, a);
+        const int c = (int)(code[f] & 7), ax = c >> 1;
+        const R sa = ax == 1 ? R(-1) : R(1);
+        const R sg = (c & 1) ? R(-1) : R(1);  // outward normal sign
+        const R w = sg * sa;
+        // J'[t2] = w H1, J'[t1] = -w H2, M[t2] = -w E1, M[t1] = w E2
+        const double j1R = (double)(-w * a[6]), j1I = (double)(-w * a[7]);
+        const double j2R = (double)(w * a[4]), j2I = (double)(w * a[5]);
+        const double m1R = (double)(w * a[2]), m1I = (double)(w * a[3]);
+        const double m2R = (double)(-w * a[0]), m2I = (double)(-w * a[1]);
+        const R x = R(pos[3 * f]), y = R(pos[3 * f + 1]), z = R(pos[3 * f + 2]);
+        double cs[kFarDirs], sn[kFarDirs];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) red[warp][q] = s[q];
+        for (int q = 0; q < kFarDirs; ++q)
+        {
+            R sr, cr;
+            sinCos(k0 * (rh[q][0] * x + rh[q][1] * y + rh[q][2] * z), &sr, &cr);
+            cs[q] = (double)cr;
+            sn[q] = (double)sr;
+        }
+        auto add = [&](auto T1, auto T2) {
+            constexpr int t1 = decltype(T1)::value, t2 = decltype(T2)::value;
+#pragma unroll
+            for (int q = 0; q < kFarDirs; ++q)
+            {
+                auto rotate = [&](int at, double re, double im) {
+                    s[q][at] = fma(re, cs[q], fma(-im, sn[q], s[q][at]));
+                    s[q][at + 1] = fma(re, sn[q], fma(im, cs[q], s[q][at + 1]));
+                };
+                rotate(2 * t1, j1R, j1I);
+                rotate(2 * t2, j2R, j2I);
+                rotate(6 + 2 * t1, m1R, m1I);
+                rotate(6 + 2 * t2, m2R, m2I);
+            }
+        };
+        using I0 = std::integral_constant<int, 0>;
+        using I1 = std::integral_constant<int, 1>;
+        using I2 = std::integral_constant<int, 2>;
+        if (ax == 0)  // faces are listed by axis: a warp takes one way
+            add(I1{}, I2{});
+        else if (ax == 1)
+            add(I0{}, I2{});
+        else
+            add(I0{}, I1{});
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < kFarDirs; ++q)
+#pragma unroll
+        for (int c = 0; c < 12; ++c)
+        {
+            double v = s[q][c];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) red[warp][q * 12 + c] = v;
+        }
+    __syncthreads();
+    if (threadIdx.x < kFarDirs * 12)
+    {
+        double v = 0;
+        for (int w = 0; w < kFarThreads / 32; ++w) v += red[w][threadIdx.x];
+        red[0][threadIdx.x] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0)
+    const int q = threadIdx.x, d = d0 + q;
+    if (q >= kFarDirs || d >= nd) return;
+    double v[12];
+#pragma unroll
+    for (int c = 0; c < 12; ++c) v[c] = red[0][q * 12 + c];
+    if (part != nullptr)
     {
-        double t[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
-            for (int q = 0; q < 8; ++q) t[q] += red[w][q];
-        const double aR = t[6] + t[0], aI = t[7] + t[1];
-        const double bR = t[4] - t[2], bI = t[5] - t[3];
-        U[d] = (R)(aR * aR + aI * aI + bR * bR + bI * bI);
+#pragma unroll
+        for (int c = 0; c < 12; ++c) part[((long long)blockIdx.y * 12 + c) * nd + d] = v[c];
     }
+    else
+        U[d] = farIntensity<R>(v, d, nTheta, nPhi);
+}
+
+template <class R>
+__global__ void __launch_bounds__(128)
+    farFieldFinish(const double *__restrict__ part, int slices, int nTheta, int nPhi, R *__restrict__ U)
+{
+    const int nd = nTheta * nPhi, d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= nd) return;
+    double v[12] = {};
+    for (int y = 0; y < slices; ++y)
+#pragma unroll
+        for (int c = 0; c < 12; ++c) v[c] += part[((long long)y * 12 + c) * nd + d];
+    U[d] = farIntensity<R>(v, d, nTheta, nPhi);
 }
 
 } // namespace tlmk
@@ -479,6 +617,8 @@ template <class S> tlm_status launchSurfaceT(tlm_solver *h, int n)
         a.scale = (R)h->scale;
         a.spec = h->dSpec;
         a.nspec = h->dSpec ? h->specCount : 0;
+        a.injLo = h->injLo;
+        a.injHi = h->injHi;
         a.sv = (R)sourceValue(h, n);
         a.jsNode = s.dJsNode;
         a.njs = nj;
@@ -512,8 +652,8 @@ template <class S> tlm_status launchSurfaceT(tlm_solver *h, int n)
         a.planeN1 = n1;
         a.planeN2 = n2;
         a.plane = static_cast<R *>(s.dPlane);
-        const long long blocks = (items + 255) / 256;
-        tlmk::surfaceMonitorKernel<S><<<(unsigned)blocks, 256, 0, h->stream>>>(a);
+        const long long blocks = (items + tlmk::kSurfaceThreads - 1) / tlmk::kSurfaceThreads;
+        tlmk::surfaceMonitorKernel<S><<<(unsigned)blocks, tlmk::kSurfaceThreads, 0, h->stream>>>(a);
         TLM_CU(h, cudaGetLastError());
         if (doPlane)
         {
@@ -577,8 +717,7 @@ tlm_status launchSurface(tlm_solver *h, int n)
 
 namespace tlmi {
 
-// Near-to-far-field transform of the Huygens phasors on the device (one block
-// per direction, FP64 sums), then the reference's directivity and peak
+// Near-to-far-field transform of the Huygens phasors on the device (FP64 sums), then the reference's directivity and peak
 // search on the host (TlmSolver.cpp:893-915). `f64`: the phasors are double.
 tlm_status farFieldTransform(cudaStream_t stream, cudaMemPool_t pool, bool f64, const void *dAcc,
                              const long long *dCode, const float *hostPos, int nh, float f0, int n_theta,
@@ -592,23 +731,36 @@ tlm_status farFieldTransform(cudaStream_t stream, cudaMemPool_t pool, bool f64, 
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&dU, (size_t)nd * r, pool, stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(dPos, hostPos, (size_t)nh * 3 * sizeof(float), cudaMemcpyHostToDevice, stream);
+    // slices of the faces, for directions too few to fill the card evenly; a
+    // slice keeps 32 faces per thread or more, and without memory for the
+    // partial sums there is one
+    const int groups = (nd + tlmk::kFarDirs - 1) / tlmk::kFarDirs;
+    int slices = std::max(1, std::min({ 4096 / groups, nh / (32 * tlmk::kFarThreads), 64 }));
+    double *dPart = nullptr;
+    if (e == cudaSuccess && slices > 1 &&
+        cudaMallocFromPoolAsync((void **)&dPart, (size_t)slices * nd * 12 * sizeof(double), pool, stream) != cudaSuccess)
+    {
+        cudaGetLastError();
+        dPart = nullptr;
+        slices = 1;
+    }
     if (e == cudaSuccess)
     {
+        auto launch = [&](auto k0) {
+            using R = decltype(k0);
+            tlmk::farFieldKernel<R><<<dim3(groups, slices), tlmk::kFarThreads, 0, stream>>>(
+                static_cast<const R *>(dAcc), dCode, dPos, nh, k0, n_theta, n_phi, static_cast<R *>(dU), dPart);
+            if (dPart)
+                tlmk::farFieldFinish<R><<<(nd + 127) / 128, 128, 0, stream>>>(dPart, slices, n_theta, n_phi,
+                                                                              static_cast<R *>(dU));
+        };
         if (f64)
-        {
-            const double k0 = 2.0 * 3.14159265358979323846 * (double)f0 / (double)299792458.0f;
-            tlmk::farFieldKernel<double><<<nd, 256, 0, stream>>>(static_cast<const double *>(dAcc), dCode, dPos,
-                                                                 nh, k0, n_theta, n_phi,
-                                                                 static_cast<double *>(dU));
-        }
+            launch(2.0 * 3.14159265358979323846 * (double)f0 / (double)299792458.0f);
         else
-        {
-            const float k0 = 2.0f * (float)3.14159265358979323846 * f0 / 299792458.0f;
-            tlmk::farFieldKernel<float><<<nd, 256, 0, stream>>>(static_cast<const float *>(dAcc), dCode, dPos, nh,
-                                                                k0, n_theta, n_phi, static_cast<float *>(dU));
-        }
+            launch(2.0f * (float)3.14159265358979323846 * f0 / 299792458.0f);
         e = cudaGetLastError();
     }
+    if (dPart) cudaFreeAsync(dPart, stream);
     std::vector<float> u(nd);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e == cudaSuccess)

@@ -1017,7 +1017,7 @@ struct fdtd_solver
     bool configured = false;
     tlm_grid g{};
     tlm_config cfg{};
-    std::vector<uint8_t> mat;
+    tlmh::HostMap mat;
     std::vector<tlm_matprops> table;
     fdk::Dims d{};
     float dt = 0, cMur = 0, cb0 = 0, ch = 0;
@@ -1698,7 +1698,8 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     const size_t n = (size_t)grid->nx * grid->ny * grid->nz;
     if (n_cells != n) return h->fail(TLM_EINVAL, "material map does not match the grid");
     // the host copy of the map and its largest id in one vectorised pass
-    std::vector<uint8_t> hostMat(n);
+    tlmh::HostMap hostMat;
+    if (!hostMat.allocate(n)) return h->fail(TLM_ENOMEM, "no host memory for the material map");
     const uint8_t maxId = tlmh::copy_max_u8(mat, hostMat.data(), n);
     if (maxId >= TLM_MAT_DIEL0 && (int)(maxId - TLM_MAT_DIEL0) >= n_table)
         return h->fail(TLM_EINVAL, "material id without a table entry");

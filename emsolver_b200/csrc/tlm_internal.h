@@ -4,6 +4,7 @@
 
 #include "tlm_b200.h"
 #include "tlm_device.cuh"
+#include "tlm_host_math.h"
 
 #include <cuda.h>
 
@@ -213,7 +214,7 @@ struct tlm_solver
     tlm_grid g{};
     tlm_config cfg{};
     int storage = TLM_STORE_F32;
-    std::vector<uint8_t> mat;
+    tlmh::HostMap mat;
     std::vector<float> epsr, sigma;
     std::vector<float> yhat32, ghat32;
     std::vector<double> yhat64, ghat64;

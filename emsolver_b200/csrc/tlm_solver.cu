@@ -313,6 +313,18 @@ template <class S> tlm_status stagedAttributes(tlm_solver *h)
     return TLM_OK;
 }
 
+// Whether single steps run their interior tiles in the staged kernel (but the
+// first one from a caller's incident pulses). FP32
+// grids below 2^20 nodes do not: there the fork and join of two kernels costs
+// more than staging gains (80x84x77 dipole 16.8 us staged, 12.6 us in one
+// kernel; 100^3 heterogeneous 26.2 and 23.8 us). A stage wait limit in the
+// configuration asks for the staged kernel.
+bool stagedStep(const tlm_solver *h)
+{
+    return h->nStaged > 0 &&
+           (h->storage != TLM_STORE_F32 || h->P >= kPairMinNodes || h->cfg.stage_wait_us != 0);
+}
+
 // FP32 with 2 nodes per thread (the default shape): interior tiles go to the
 // staged kernel, the others (PEC, sources, monitors, the partial last tile)
 // to the list kernel, both launched every step (tlm_config.no_staging = 1: the single
@@ -367,35 +379,42 @@ tlm_status prepareStaging(tlm_solver *h, const std::vector<uint8_t> &flags)
             return TLM_OK;
         }
     }
-    int sms = 0;
-    TLM_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    if (h->storage == TLM_STORE_F16)
-        TLM_TRY(stagedAttributes<__half>(h));
-    else if (h->storage == TLM_STORE_BF16)
-        TLM_TRY(stagedAttributes<__nv_bfloat16>(h));
-    else
-        TLM_TRY(stagedAttributes<float>(h));
-    if (!h->side)
-    {
-        TLM_CU(h, cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-        TLM_CU(h, cudaEventCreateWithFlags(&h->evFork, cudaEventDisableTiming));
-        TLM_CU(h, cudaEventCreateWithFlags(&h->evJoin, cudaEventDisableTiming));
-    }
-    TLM_TRY(devAlloc(h, &h->dStaged, staged.size() * sizeof(int)));
-    TLM_CU(h, cudaMemcpyAsync(h->dStaged, staged.data(), staged.size() * sizeof(int), cudaMemcpyHostToDevice,
-                              h->stream));
-    if (!listed.empty())
-    {
-        TLM_TRY(devAlloc(h, &h->dListed, listed.size() * sizeof(int)));
-        TLM_CU(h, cudaMemcpyAsync(h->dListed, listed.data(), listed.size() * sizeof(int), cudaMemcpyHostToDevice,
-                                  h->stream));
-    }
     h->nStaged = (int)staged.size();
-    for (int e : staged) h->sparseStaged |= (tlmk::entryFlags(e) & tlmk::kTileStubSparse) != 0;
     h->nListed = (int)listed.size();
+    // (a batch reads the host lists: what only launches of the staged kernel
+    // need, the device lists and a second stream, is made for handles that
+    // launch it; without them a small grid's first step and its close take 180
+    // instead of 340 us)
+    if (stagedStep(h))
+    {
+        int sms = 0;
+        TLM_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+        if (h->storage == TLM_STORE_F16)
+            TLM_TRY(stagedAttributes<__half>(h));
+        else if (h->storage == TLM_STORE_BF16)
+            TLM_TRY(stagedAttributes<__nv_bfloat16>(h));
+        else
+            TLM_TRY(stagedAttributes<float>(h));
+        if (!h->side)
+        {
+            TLM_CU(h, cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+            TLM_CU(h, cudaEventCreateWithFlags(&h->evFork, cudaEventDisableTiming));
+            TLM_CU(h, cudaEventCreateWithFlags(&h->evJoin, cudaEventDisableTiming));
+        }
+        TLM_TRY(devAlloc(h, &h->dStaged, staged.size() * sizeof(int)));
+        TLM_CU(h, cudaMemcpyAsync(h->dStaged, staged.data(), staged.size() * sizeof(int), cudaMemcpyHostToDevice,
+                                  h->stream));
+        if (!listed.empty())
+        {
+            TLM_TRY(devAlloc(h, &h->dListed, listed.size() * sizeof(int)));
+            TLM_CU(h, cudaMemcpyAsync(h->dListed, listed.data(), listed.size() * sizeof(int), cudaMemcpyHostToDevice,
+                                      h->stream));
+        }
+        h->stagedGrid = std::min(h->nStaged, 2 * sms);
+    }
+    for (int e : staged) h->sparseStaged |= (tlmk::entryFlags(e) & tlmk::kTileStubSparse) != 0;
     h->stagedTiles = std::move(staged);
     h->listedTiles = std::move(listed);
-    h->stagedGrid = std::min(h->nStaged, 2 * sms);
     return TLM_OK;
 }
 
@@ -659,17 +678,6 @@ tlm_status timeLaunch(tlm_solver *h, int steps, cudaEvent_t *after)
     return TLM_OK;
 }
 
-// Whether a single step runs its interior tiles in the staged kernel. FP32
-// grids below 2^20 nodes do not: there the fork and join of two kernels costs
-// more than staging gains (80x84x77 dipole 16.8 us staged, 12.6 us in one
-// kernel; 100^3 heterogeneous 26.2 and 23.8 us). A stage wait limit in the
-// configuration asks for the staged kernel.
-bool stagedStep(const tlm_solver *h)
-{
-    return h->nStaged > 0 && !h->stateIncident &&
-           (h->storage != TLM_STORE_F32 || h->P >= kPairMinNodes || h->cfg.stage_wait_us != 0);
-}
-
 template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long eFirst)
 {
     const tlmk::StepArgs<S> a = stepArgs<S>(h, n, i, eFirst);
@@ -678,7 +686,7 @@ template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long 
     if (surfaceActive(h)) TLM_TRY(launchSurface(h, n));  // reads the same input buffer, first
     if constexpr (std::is_same<S, float>::value)
     {
-        if (stagedStep(h))
+        if (stagedStep(h) && !h->stateIncident)
         {
             // the listed tiles run beside the staged ones (disjoint outputs,
             // the same input), on the side stream between a fork and a join
@@ -704,7 +712,7 @@ template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long 
     }
     else if constexpr (std::is_same<S, __half>::value || std::is_same<S, __nv_bfloat16>::value)
     {
-        if (stagedStep(h))
+        if (stagedStep(h) && !h->stateIncident)
         {
             // as FP32: the listed tiles beside the staged ones
             if (h->nListed > 0)
@@ -1657,7 +1665,8 @@ tlm_status tlm_setup(tlm_handle h, const tlm_grid *grid, const uint8_t *mat, siz
     // (tlm_host_math.cpp, built by g++; the same scan compiled here measured
     // 3.9 ms on 192^3); the largest id decides, and the first offending cell
     // is looked for only when there is one
-    std::vector<uint8_t> hostMat((size_t)n);
+    tlmh::HostMap hostMat;
+    if (!hostMat.allocate((size_t)n)) return h->fail(TLM_ENOMEM, "no host memory for the material map");
     const uint8_t maxId = tlmh::copy_max_u8(mat, hostMat.data(), (size_t)n);
     const bool anyDiel = maxId >= TLM_MAT_DIEL0;
     if (anyDiel && maxId - TLM_MAT_DIEL0 >= n_table)
@@ -2624,7 +2633,7 @@ tlm_status tlm_step_launches(tlm_handle h, int *per_step)
     TLM_TRY(checkHandle(h));
     if (!per_step) return h->fail(TLM_EINVAL, "null output");
     TLM_TRY(prepare(h));
-    *per_step = (stagedStep(h) ? (h->nListed > 0 ? 2 : 1) : 1) + (surfaceActive(h) ? 1 : 0);
+    *per_step = (stagedStep(h) && !h->stateIncident ? (h->nListed > 0 ? 2 : 1) : 1) + (surfaceActive(h) ? 1 : 0);
     return TLM_OK;
 }
 

@@ -13,8 +13,8 @@
 // caller's n_diel entries read NaN there instead of reading past the caller's
 // buffers), and the last block to finish adds up the blocks' energies in a
 // fixed order. The only scratch, an FP64 partial per block and the count of
-// finished blocks, lives in the file-scope arrays below, a fixed 16 KiB of
-// device memory that every GPU which loads this library holds until the
+// finished blocks, 16 slots of them, lives in the file-scope arrays below, a fixed
+// 74 KiB of device memory that every GPU which loads this library holds until the
 // process exits. Host code must not pass an array's name to a kernel (on the
 // host that name is a stand-in, not a device address); the device addresses
 // are looked up once per device with cudaGetSymbolAddress.
@@ -23,6 +23,7 @@
 #include "tlm_pair_kernel.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <string>
 
@@ -32,9 +33,9 @@ void tlmSetThreadError(const std::string &m);
 
 // The grid is limited to 67,108,864 padded nodes (2^25 pairs).
 constexpr long long kNoAllocMaxNodes = 67108864;
-constexpr int kNoAllocMaxBlocks = 2048;
-static __device__ __align__(256) double g_noallocPartials[kNoAllocMaxBlocks];
-static __device__ __align__(256) unsigned g_noallocDone;
+constexpr int kNoAllocMaxBlocks = 148 * 4, kNoAllocSlots = 16;
+static __device__ __align__(256) double g_noallocPartials[kNoAllocSlots * kNoAllocMaxBlocks];
+static __device__ __align__(256) unsigned g_noallocDone[kNoAllocSlots];
 constexpr int kNoAllocTable = 256 - tlmk::kDiel0;
 // Bounds-check record of the checked library build (cleared before every
 // step, read back after it there); the regular build never writes it.
@@ -44,6 +45,7 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 std::mutex g_noallocMutex;
+std::atomic<unsigned> g_noallocCalls{ 0 };
 
 struct NoAllocScratch
 {
@@ -329,13 +331,15 @@ tlm_status tlm_step_planes_noalloc(const float *in_planes, float *out_planes, fl
     a.divY = tlmk::makeFastDiv((unsigned)ny);
     a.rho = rho;
     a.neg_zero = -0.0f;
-    a.partials = sc.partials;
+    // calls take the slots in turn, so that a few which overlap on the GPU keep
+    // apart
+    const unsigned slot = g_noallocCalls.fetch_add(1) % kNoAllocSlots;
+    a.partials = sc.partials + slot * kNoAllocMaxBlocks;
     a.energy = energy_out;
-    a.done = sc.done;
+    a.done = sc.done + slot;
     a.fault = sc.fault;
     // four resident blocks per SM walk over the tiles of large grids
-    const unsigned blocks = std::min((a.npairs + 255u) / 256u, 148u * 4u);
-    static_assert(148 * 4 <= kNoAllocMaxBlocks, "a partial per block");
+    const unsigned blocks = std::min((a.npairs + 255u) / 256u, (unsigned)kNoAllocMaxBlocks);
     if (input_is_incident)
     {
         if (stubs) planesStepKernel<true, true><<<blocks, 256, 0, s>>>(a);

@@ -555,14 +555,15 @@ TLM_API tlm_status tlm_get_halo_stream(tlm_handle h, void **stream);
  * Work is queued on `stream` (a cudaStream_t, NULL = default stream).
  *
  * Limits and sharing: its only scratch, one FP64 energy partial per thread
- * block and a count of finished blocks, is a fixed 16 KiB of static device
+ * block and a count of finished blocks, is 16 slots in a fixed 74 KiB of static device
  * arrays that every GPU loading this library holds until the process exits;
  * grids above 67,108,864 padded nodes are rejected with TLM_EINVAL. The
  * first call on a device looks up those arrays' device addresses
  * (cudaGetSymbolAddress); make that first call before any stream capture.
- * Every call shares the arrays, so calls that overlap on the GPU (other
- * streams, other threads) race: serialise them. Each call rewrites the
- * partials it uses and leaves the count at zero; nothing needs clearing. The bounds-checked build
+ * Calls take the slots in turn: of calls that overlap on the GPU (other
+ * streams, other threads) at most 16 in a row keep apart, and a captured call
+ * keeps its slot in every replay; serialise what goes beyond that. Each call
+ * rewrites the partials it uses and leaves the count at zero. The bounds-checked build
  * of the library (libtlm_b200_checked.so) waits for the step and returns
  * TLM_ECUDA if any index fell outside its buffer.
  * Errors: status code, message in tlm_last_error(NULL). */

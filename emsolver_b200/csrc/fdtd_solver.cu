@@ -14,8 +14,9 @@
 //      order reproduces the reference's six face passes (edges shared by two
 //      faces end with the later pass's value).
 // Steps 3 and 4 are one pass over memory (fusedStepKernel) from one field
-// buffer to another, and a Mur kernel that takes the old boundary values from
-// the input buffer; without room for a second field buffer they run in place,
+// buffer to another, then a tail kernel (stepTailKernel): Mur, which takes the
+// old boundary values from the input buffer, the monitors, and the next step's
+// sources; without room for a second field buffer they run in place,
 // one sweep for H and one for E.
 // Fields: one plane set per component, all six with the same pitch (cell
 // (i, j, k) of every component at (k*(ny+1) + j)*px + i; entries that a

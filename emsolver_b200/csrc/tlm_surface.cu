@@ -157,12 +157,11 @@ template <class R, int N> __device__ __forceinline__ void storeAcc(R *p, const R
 
 // One thread per face or cut-plane point. Bound by the chain of dependent
 // loads (a face touches 12 pulses, 6 materials and its accumulators, scattered
-// for x faces, and the faces of a 96^3 Huygens box fill a third of the
+// for x faces, and the 38,688 faces of a 104x96x101 grid fill an eighth of the
 // card's threads), so the chain is kept at two: the face's code and
 // accumulators, then everything else; only a PEC neighbour and a face among the
 // sources add one.
-// On a B200, 48,600 Huygens faces of a 96^3 grid, FP32, caches cold: 20.0 ->
-// 8.5 us per step.
+// On a B200, those faces, FP32, caches cold: 20.0 -> 8.5 us per step.
 template <class S> __global__ void __launch_bounds__(kSurfaceThreads) surfaceMonitorKernel(const SurfaceArgs<S> a)
 {
     using R = typename Traits<S>::R;
@@ -259,7 +258,7 @@ template <class S> __global__ void __launch_bounds__(kSurfaceThreads) surfaceMon
 // Sums run in a fixed order: a thread's faces, lanes, warps, slices. With more
 // than one slice the blocks leave their sums in `part` for farFieldFinish.
 // Bound by issue (sine, cosine and 16 FP64 operations per face and direction).
-// 37 x 73 directions of 48,600 FP32 faces on a B200: 1584 -> 421 us (one block of
+// 37 x 73 directions of 38,688 FP32 faces on a B200: 1584 -> 421 us (one block of
 // 256 threads per direction, its projections summed, before).
 constexpr int kFarDirs = 4, kFarThreads = 128;
 

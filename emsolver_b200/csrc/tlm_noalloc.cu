@@ -177,12 +177,27 @@ template <bool INCIDENT, bool DIEL> __global__ void __launch_bounds__(256, 4) pl
         float2 o[12];
         if (DIEL && (word & kMatDiel))
         {
+            // the caller's stubs count on dielectric nodes only: the other node
+            // of a pair may hold anything there, and keeps it
+            const bool d0 = word & (1u << 16), d1 = word & (2u << 16);
             float2 vs[3];
 #pragma unroll
-            for (int t = 0; t < 3; ++t) vs[t] = ld2(a.stub + t * P + n0);
+            for (int t = 0; t < 3; ++t)
+            {
+                vs[t] = ld2(a.stub + t * P + n0);
+                if (!d0) vs[t].x = 0.0f;
+                if (!d1) vs[t].y = 0.0f;
+            }
             pairScatterStub(tab, inc, vs, word, z, o);
 #pragma unroll
-            for (int t = 0; t < 3; ++t) *reinterpret_cast<float2 *>(a.stub + t * P + n0) = vs[t];
+            for (int t = 0; t < 3; ++t)
+            {
+                float *w = a.stub + t * P + n0;
+                if (d0 && d1)
+                    *reinterpret_cast<float2 *>(w) = vs[t];
+                else
+                    w[d1 ? 1 : 0] = d1 ? vs[t].y : vs[t].x;
+            }
         }
         else
         {

@@ -217,6 +217,7 @@ struct tlm_solver
     tlmh::HostMap mat;
     std::vector<float> epsr, sigma;
     std::vector<float> yhat32, ghat32;
+    float divLimit = 0.0f;  // of the FP32 tables (tlmk::stubDivLimit)
     std::vector<double> yhat64, ghat64;
     int nx = 0, ny = 0, nz = 0, px = 0, V = 4, nq = 0;
     long long P = 0, ncell = 0, nquads = 0;

@@ -89,19 +89,25 @@ template <bool INCIDENT, bool DIEL> __global__ void __launch_bounds__(256, 4) pl
     __shared__ float tab[768];
     __shared__ double red[8];
     __shared__ bool lastBlock;
+    float divLimit = 0.0f;
     if constexpr (DIEL)
     {
-        for (int m = threadIdx.x; m < 256; m += 256)
-        {
-            const float nan = __int_as_float(0x7fc00000);
-            const float yh = m < kDiel0 ? -0.0f : m - kDiel0 < a.ntable ? a.yhat[m - kDiel0] : nan;
-            const float gh = m < kDiel0 ? 0.0f : m - kDiel0 < a.ntable ? a.ghat[m - kDiel0] : nan;
-            const float den = (4.0f + yh) + gh;
-            tab[m] = yh;
-            tab[256 + m] = -den;
-            tab[512 + m] = __frcp_rn(den);
-        }
-        __syncthreads();
+        static_assert(kBlock == 256, "a thread per material id");
+        const int m = threadIdx.x;
+        const float nan = __int_as_float(0x7fc00000);
+        const bool in = m >= kDiel0 && m - kDiel0 < a.ntable;
+        const float yh = m < kDiel0 ? -0.0f : in ? a.yhat[m - kDiel0] : nan;
+        const float gh = m < kDiel0 ? 0.0f : in ? a.ghat[m - kDiel0] : nan;
+        const float den = (4.0f + yh) + gh;
+        tab[m] = yh;
+        tab[256 + m] = -den;
+        tab[512 + m] = __frcp_rn(den);
+        // the limit of the caller's denominators, which may be anything, in
+        // steps: at most 2^25, at most 2^40, or out of range (also below 4)
+        const bool low = den >= 4.0f;
+        divLimit = stubDivLimit(4.0f);
+        if (__syncthreads_or(in && !(low && den <= 0x1p25f)))
+            divLimit = stubDivLimit(__syncthreads_or(in && !(low && den <= 0x1p40f)) ? nan : 0x1p40f);
     }
     const long long P = a.P, sz = (long long)a.px * a.ny;
     const float2 z = splat2(a.neg_zero), rho = splat2(a.rho);
@@ -188,7 +194,7 @@ template <bool INCIDENT, bool DIEL> __global__ void __launch_bounds__(256, 4) pl
                 if (!d0) vs[t].x = 0.0f;
                 if (!d1) vs[t].y = 0.0f;
             }
-            pairScatterStub(tab, inc, vs, word, z, o);
+            pairScatterStub(tab, inc, vs, word, divLimit, z, o);
 #pragma unroll
             for (int t = 0; t < 3; ++t)
             {

@@ -43,6 +43,8 @@
 
 #include "tlm_step_kernel.cuh"
 
+#include <cmath>
+
 namespace tlmk {
 
 
@@ -94,6 +96,7 @@ struct PairArgs
     float *stubOut;
     const float *yhat, *ghat;
     int ntable;
+    float divLimit;                // stubDivLimit of the material table
     const unsigned *flags;         // [column][nz]
     long long P;
     int nx, ny, nz, px;
@@ -186,7 +189,18 @@ __device__ __forceinline__ unsigned matWord(unsigned ids, unsigned dead)
 // correction q is within an ulp of the quotient, so the residual is exact and
 // the second one rounds correctly (P. Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990),
-// as long as nothing under- or overflows: 2^-100 < |n| < 2^120.
+// as long as nothing under- or overflows: |n| < 2^120, and above the table's limit
+// (stubDivLimit), so that the quotient is normal.
+//
+// The limit for a table whose denominators, 4 or more, reach denMax: 2^-100, for a
+// denominator above 2^25 as much more as keeps the quotient above 2^-125, and
+// infinity (every pair divides as IEEE does) above 2^40, where a quotient of
+// scaled numerators may be subnormal as well, and for infinities and NaN.
+__host__ __device__ __forceinline__ float stubDivLimit(float denMax)
+{
+    if (!(denMax <= 0x1p40f)) return HUGE_VALF;
+    return denMax <= 0x1p25f ? 0x1p-100f : denMax * 0x1p-125f;
+}
 __device__ __forceinline__ void divByTable(const float2 (&num)[3], float2 nden, float2 rcp, float2 z, float2 (&q)[3])
 {
 #pragma unroll
@@ -207,9 +221,10 @@ __device__ __forceinline__ void divByTable(const float2 (&num)[3], float2 nden, 
 // where q is a tie of the subnormal grid but not the exact quotient: there q
 // moves an ulp towards the exact quotient, on the side its residual tells. A
 // zero quotient has the numerator's sign (den > 0). Lanes with numerators of
-// 2^40 and more beside tiny ones take the IEEE division.
+// 2^40 and more beside tiny ones take the IEEE division, and so do all where
+// `limit` (stubDivLimit) is infinite.
 __device__ __forceinline__ void pairScatterStub(const float *tab, const float2 (&in)[12], float2 (&vs)[3], unsigned m,
-                                                float2 z, float2 (&out)[12])
+                                                float limit, float2 z, float2 (&out)[12])
 {
     const unsigned diel = (m & kMatDiel) >> 16;
     const float *t0 = tab + (m & 255u), *t1 = tab + ((m >> 8) & 255u);
@@ -228,14 +243,14 @@ __device__ __forceinline__ void pairScatterStub(const float *tab, const float2 (
         lo = fminf(lo, fminf(fabsf(num[j].x), fabsf(num[j].y)));
         hi = fmaxf(hi, fmaxf(fabsf(num[j].x), fabsf(num[j].y)));
     }
-    if (lo > 0x1p-100f && hi < 0x1p120f)
+    if (lo > limit && hi < 0x1p120f)
         divByTable(num, nden, rcp, z, Vn);
-    else if (hi == 0.0f)
+    else if (hi == 0.0f && limit < 1.0f)
     {
 #pragma unroll
         for (int j = 0; j < 3; ++j) Vn[j] = num[j];
     }
-    else if (hi < 0x1p40f)
+    else if (hi < 0x1p40f && limit < 1.0f)
     {
         // distance of each scaled quotient from the value it scales back to
         auto off = [&](float2 q) { return sub2(q, mul2(mul2(q, splat2(0x1p-64f), z), splat2(0x1p64f), z)); };
@@ -421,7 +436,7 @@ __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks) stepPairKernel(con
     auto scatter = [&](unsigned lanes, unsigned f, const float2(&inc)[12], float2(&vs)[3], unsigned m,
                        float2(&out)[12]) {
         if (DIEL && (f & kPairDiel) && __any_sync(lanes, (m & kMatDiel) != 0))
-            pairScatterStub(tab, inc, vs, m, negZero, out);
+            pairScatterStub(tab, inc, vs, m, a.divLimit, negZero, out);
         else
             scatterAir2(inc, out, negZero);
     };

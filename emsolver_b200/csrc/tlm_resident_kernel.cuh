@@ -52,6 +52,7 @@ struct ResidentArgs
     const uint8_t *mat;
     const float *yhat, *ghat;
     int ntable;
+    float divLimit;           // stubDivLimit of the material table
     long long P;
     int nx, ny, nz, px;
     int by, bz, gy, gz;       // rows and planes per brick (2 or more, or all), bricks in y and z
@@ -390,7 +391,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentKernel(const __gr
             float2 vs[3];
 #pragma unroll
             for (int t = 0; t < 3; ++t) vs[t] = ld2(stubs + t * L::SS + at[m]);
-            pairScatterStub(tab, inc, vs, word[m], z, o);
+            pairScatterStub(tab, inc, vs, word[m], a.divLimit, z, o);
 #pragma unroll
             for (int t = 0; t < 3; ++t) *reinterpret_cast<float2 *>(stubs + t * L::SS + at[m]) = vs[t];
         }

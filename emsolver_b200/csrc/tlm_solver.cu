@@ -910,6 +910,7 @@ tlm_status launchPair(tlm_solver *h, int n, int i, long long eFirst)
     a.yhat = s0.yhat;
     a.ghat = s0.ghat;
     a.ntable = (int)h->epsr.size();
+    a.divLimit = h->divLimit;
     a.flags = h->dPairFlags;
     a.P = h->P;
     a.nx = h->nx;
@@ -1044,6 +1045,7 @@ tlm_status launchResident(tlm_solver *h, int n, int i, int steps, long long eFir
     a.yhat = static_cast<const float *>(h->dYhat);
     a.ghat = static_cast<const float *>(h->dGhat);
     a.ntable = (int)h->epsr.size();
+    a.divLimit = h->divLimit;
     a.P = h->P;
     a.nx = h->nx;
     a.ny = h->ny;
@@ -1713,6 +1715,14 @@ tlm_status tlm_setup(tlm_handle h, const tlm_grid *grid, const uint8_t *mat, siz
                      h->ghat32.data());
     tlmh::tables_f64(h->epsr.data(), h->sigma.data(), n_table, grid->dl, h->yhat64.data(),
                      h->ghat64.data());
+    float denMax = 4.0f;
+    for (int t = 0; t < n_table; ++t)
+    {
+        const float den = (4.0f + h->yhat32[t]) + h->ghat32[t];
+        denMax = den <= 0x1p40f ? std::max(denMax, den) : HUGE_VALF;
+        if (denMax > 0x1p40f) break;
+    }
+    h->divLimit = tlmk::stubDivLimit(denMax);
     h->dt32 = tlmh::timestep_f32(grid->dl);
     h->dt64 = tlmh::timestep_f64(grid->dl);
     h->sources.clear();

@@ -1756,9 +1756,10 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     // coefficients of the edges inside one material: the sums over four equal cells
     std::vector<float2> tab(fdk::kEdgeClasses, make_float2(0.0f, 0.0f)), props(std::max(n_table, 1), make_float2(1.0f, 0.0f));
     tab[fdk::kEdgeAir] = make_float2(1.0f, h->cb0);
-    for (int t = 0; t < n_table; ++t)
+    for (int t = 0; t < n_table; ++t) props[t] = make_float2(table[t].epsr, table[t].sigma);
+    // (a byte names 254 dielectrics; no cell can have a later entry)
+    for (int t = 0; t < std::min(n_table, (int)fdk::kEdgeFirst - TLM_MAT_DIEL0); ++t)
     {
-        props[t] = make_float2(table[t].epsr, table[t].sigma);
         const int id = t + TLM_MAT_DIEL0;
         const float e1 = 1.0f + (table[t].epsr - 1.0f), s1 = table[t].sigma;
         float e = 0.0f, sg = 0.0f;

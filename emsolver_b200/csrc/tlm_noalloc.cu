@@ -35,7 +35,7 @@ void tlmSetThreadError(const std::string &m);
 constexpr long long kNoAllocMaxNodes = 67108864;
 constexpr int kNoAllocMaxBlocks = 148 * 4, kNoAllocSlots = 16;
 static __device__ __align__(256) double g_noallocPartials[kNoAllocSlots * kNoAllocMaxBlocks];
-static __device__ __align__(256) unsigned g_noallocDone[kNoAllocSlots];
+static __device__ __align__(256) unsigned long long g_noallocDone[kNoAllocSlots];
 constexpr int kNoAllocTable = 256 - tlmk::kDiel0;
 // Bounds-check record of the checked library build (cleared before every
 // step, read back after it there); the regular build never writes it.
@@ -45,12 +45,12 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 std::mutex g_noallocMutex;
-std::atomic<unsigned> g_noallocCalls{ 0 };
+std::atomic<unsigned long long> g_noallocCalls{ 0 };
 
 struct NoAllocScratch
 {
     double *partials = nullptr;
-    unsigned *done = nullptr;
+    unsigned long long *done = nullptr;
     unsigned *fault = nullptr;
 };
 NoAllocScratch g_noallocAddr[kMaxDevices];
@@ -74,7 +74,8 @@ struct PlanesArgs
     tlmk::FastDiv divH, divY;  // by hx and by ny
     float rho, neg_zero;
     double *partials, *energy;
-    unsigned *done, *fault;
+    unsigned long long *done, call;  // finished blocks of this call: call + their number
+    unsigned *fault;
 };
 
 // One step, a pair of nodes per thread at a time, the arithmetic of the general
@@ -237,7 +238,10 @@ template <bool INCIDENT, bool DIEL> __global__ void __launch_bounds__(256, 4) pl
     {
         a.partials[blockIdx.x] = tot;
         __threadfence();
-        lastBlock = atomicAdd(a.done, 1u) == gridDim.x - 1;
+        // whatever an earlier call left in the count, this call's begins at
+        // its own number, which is larger
+        atomicMax(a.done, a.call);
+        lastBlock = atomicAdd(a.done, 1ull) == a.call + gridDim.x - 1;
     }
     __syncthreads();
     if (!lastBlock) return;
@@ -246,11 +250,7 @@ template <bool INCIDENT, bool DIEL> __global__ void __launch_bounds__(256, 4) pl
     for (unsigned b = threadIdx.x; b < gridDim.x; b += 256) s += __ldcg(a.partials + b);
     __syncthreads();
     const double all = blockSumDouble(s, red);
-    if (threadIdx.x == 0)
-    {
-        *a.energy = all;
-        *a.done = 0;
-    }
+    if (threadIdx.x == 0) *a.energy = all;
 }
 
 // Device addresses of the scratch arrays for the current device, looked up
@@ -279,7 +279,7 @@ tlm_status scratchForCurrentDevice(NoAllocScratch *out)
             return noallocFail(TLM_ECUDA, std::string("cudaGetSymbolAddress of the scratch arrays: ") +
                                               cudaGetErrorString(e));
         }
-        sc.done = static_cast<unsigned *>(t);
+        sc.done = static_cast<unsigned long long *>(t);
         sc.fault = static_cast<unsigned *>(f);
         sc.partials = static_cast<double *>(p);
     }
@@ -353,11 +353,25 @@ tlm_status tlm_step_planes_noalloc(const float *in_planes, float *out_planes, fl
     a.rho = rho;
     a.neg_zero = -0.0f;
     // calls take the slots in turn, so that a few which overlap on the GPU keep
-    // apart
-    const unsigned slot = g_noallocCalls.fetch_add(1) % kNoAllocSlots;
+    // apart; what a collision beyond that leaves in a count harms no later call,
+    // whose number is larger (in a captured call's replays it is always the same
+    // one: they clear the count first)
+    const unsigned long long call = g_noallocCalls.fetch_add(1) + 1;
+    const unsigned slot = (unsigned)(call % kNoAllocSlots);
     a.partials = sc.partials + slot * kNoAllocMaxBlocks;
     a.energy = energy_out;
     a.done = sc.done + slot;
+    a.call = call << 16;  // room for the blocks of many overlapping calls
+    if (energy_out)
+    {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &capture) != cudaSuccess)
+            cudaGetLastError();
+        else if (capture == cudaStreamCaptureStatusActive)
+            e = cudaMemsetAsync(a.done, 0, sizeof(*a.done), s);
+        if (e != cudaSuccess)
+            return noallocFail(TLM_ECUDA, std::string("no-allocation step set-up: ") + cudaGetErrorString(e));
+    }
     a.fault = sc.fault;
     // four resident blocks per SM walk over the tiles of large grids
     const unsigned blocks = std::min((a.npairs + 255u) / 256u, (unsigned)kNoAllocMaxBlocks);

@@ -562,8 +562,9 @@ TLM_API tlm_status tlm_get_halo_stream(tlm_handle h, void **stream);
  * (cudaGetSymbolAddress); make that first call before any stream capture.
  * Calls take the slots in turn: of calls that overlap on the GPU (other
  * streams, other threads) at most 16 in a row keep apart, and a captured call
- * keeps its slot in every replay; serialise what goes beyond that. Each call
- * rewrites the partials it uses and leaves the count at zero. The bounds-checked build
+ * keeps its slot in every replay; serialise what goes beyond that, or the
+ * energy_out of the calls that collide is undefined (their pulses and stubs are
+ * not, nor anything of later calls). The bounds-checked build
  * of the library (libtlm_b200_checked.so) waits for the step and returns
  * TLM_ECUDA if any index fell outside its buffer.
  * Errors: status code, message in tlm_last_error(NULL). */

@@ -361,7 +361,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentKernel(const __gr
                         if (a.spec[mid].node < (long long)node[m]) lo = mid + 1; else hi = mid;
                     }
                 }
-                for (int e = 0; e < (int)(spec[m] & 0xffffu); ++e)
+                const int n = (int)(spec[m] & (listed ? 0xffffu : 0x7fffffffu));
+                for (int e = 0; e < n; ++e)
                 {
                     SpecEntry se;
                     bool sec;

@@ -293,6 +293,7 @@ struct tlm_solver
     // pass writes (swapped with dStub after every pass)
     std::shared_ptr<tlmi::PairPlan> pair;
     bool pairTried = false;
+    size_t pairBytes = 0;                // device bytes of the plan
     unsigned *dPairFlags = nullptr;
     unsigned *dPairWord = nullptr;       // material word of every node pair
     int *dSpecRow = nullptr;             // first entry of dSpec in every row of nodes
@@ -359,12 +360,25 @@ namespace tlmi {
 // Device memory of a handle comes from a per-device stream-ordered pool that
 // keeps freed blocks for reuse (no device-wide synchronisation and no
 // driver round trip per allocation), ordered on the handle's stream.
+// What a handle can do without (the plan of two-step passes) is given up for
+// what it cannot: true if there was anything.
+bool reclaim(tlm_solver *h);
+inline cudaError_t poolAlloc(tlm_solver *h, void **q, size_t bytes)
+{
+    cudaError_t e = cudaMallocFromPoolAsync(q, bytes, h->pool, h->stream);
+    if (e == cudaErrorMemoryAllocation && reclaim(h))
+    {
+        cudaGetLastError();
+        e = cudaMallocFromPoolAsync(q, bytes, h->pool, h->stream);
+    }
+    return e;
+}
 template <class T> tlm_status devAlloc(tlm_solver *h, T **p, size_t bytes)
 {
     *p = nullptr;
     if (bytes == 0) return TLM_OK;
     void *q = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&q, bytes, h->pool, h->stream);
+    cudaError_t e = poolAlloc(h, &q, bytes);
     if (e != cudaSuccess)
     {
         cudaGetLastError();
@@ -379,7 +393,7 @@ template <class T> tlm_status devAlloc(tlm_solver *h, T **p, size_t bytes)
 template <class T> tlm_status tmpAlloc(tlm_solver *h, T **p, size_t bytes)
 {
     void *q = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&q, bytes > 0 ? bytes : 1, h->pool, h->stream);
+    cudaError_t e = poolAlloc(h, &q, bytes > 0 ? bytes : 1);
     if (e != cudaSuccess)
     {
         cudaGetLastError();

@@ -59,8 +59,34 @@ namespace tlmi {
 
 
 
+// Forget the plan of two-step passes (or what a failed attempt at one has
+// allocated so far) with its memory; the next step may plan again.
+void dropPair(tlm_solver *h)
+{
+    h->pair.reset();
+    h->pairTried = false;
+    devFree(h, h->dPairFlags);
+    devFree(h, h->dPairWord);
+    devFree(h, h->dSpecRow);
+    devFree(h, h->dStubAlt);
+    devFree(h, h->dEpair);
+    h->devBytes -= h->pairBytes;
+    h->pairBytes = 0;
+}
+
+bool reclaim(tlm_solver *h)
+{
+    if (!h->pair) return false;
+    dropPair(h);
+    // the blocks go back to the device: the pool does not join them into a larger one
+    cudaStreamSynchronize(h->stream);
+    cudaMemPoolTrimTo(h->pool, 0);
+    return true;
+}
+
 void freeMonitors(tlm_solver *h)
 {
+    dropPair(h);
     freeSurface(h);
     devFree(h, h->dSpec);
     devFree(h, h->dTile);
@@ -68,12 +94,6 @@ void freeMonitors(tlm_solver *h)
     devFree(h, h->dStaged);
     devFree(h, h->dListed);
     h->nStaged = h->nListed = 0;
-    h->pair.reset();
-    h->pairTried = false;
-    devFree(h, h->dPairFlags);
-    devFree(h, h->dPairWord);
-    devFree(h, h->dSpecRow);
-    devFree(h, h->dStubAlt);
     h->resTried = false;
     h->resBy = 0;
     devFree(h, h->dResPack);
@@ -809,13 +829,10 @@ TensorMapEncoder tensorMapEncoder()
     return fn;
 }
 
-// Plan the two-step passes of a handle, once per prepare; without one (not
-// enough memory for the second set of stub planes, no tensor maps) the handle
-// keeps stepping one step per launch.
-tlm_status ensurePair(tlm_solver *h)
+// Plan the two-step passes of a handle (h->pair stays null where they are not
+// possible).
+static tlm_status planPair(tlm_solver *h)
 {
-    if (h->pairTried) return TLM_OK;
-    h->pairTried = true;
     TensorMapEncoder encode = tensorMapEncoder();
     if (!encode) return TLM_OK;
     {
@@ -857,10 +874,10 @@ tlm_status ensurePair(tlm_solver *h)
     });
     TLM_TRY(st);
     if (!ok) return TLM_OK;
-    if (!h->dEpair && devAlloc(h, &h->dEpair, (size_t)(h->P / 2) * sizeof(double)) != TLM_OK) return TLM_OK;
+    TLM_TRY(devAlloc(h, &h->dEpair, (size_t)(h->P / 2) * sizeof(double)));
     if (h->dStub)
     {
-        if (devAlloc(h, &h->dStubAlt, 3 * (size_t)h->P * sizeof(float)) != TLM_OK) return TLM_OK;
+        TLM_TRY(devAlloc(h, &h->dStubAlt, 3 * (size_t)h->P * sizeof(float)));
         TLM_CU(h, cudaMemsetAsync(h->dStubAlt, 0, 3 * (size_t)h->P * sizeof(float), h->stream));
     }
     const size_t nf = (size_t)g.ntx * g.nty * h->nz;
@@ -868,9 +885,8 @@ tlm_status ensurePair(tlm_solver *h)
     TLM_CU(h, cudaMemsetAsync(h->dPairFlags, 0, nf * sizeof(unsigned), h->stream));
     tlmk::pairMaterialFlags<<<(unsigned)nf, 128, 0, h->stream>>>(h->dMat, h->nx, h->ny, h->nz, h->px, g, h->dPairFlags);
     const long long npairs = h->P / 2, rows = (long long)h->ny * h->nz;
-    if (devAlloc(h, &h->dPairWord, (size_t)npairs * sizeof(unsigned)) != TLM_OK ||
-        devAlloc(h, &h->dSpecRow, (size_t)(rows + 1) * sizeof(int)) != TLM_OK)
-        return TLM_OK;
+    TLM_TRY(devAlloc(h, &h->dPairWord, (size_t)npairs * sizeof(unsigned)));
+    TLM_TRY(devAlloc(h, &h->dSpecRow, (size_t)(rows + 1) * sizeof(int)));
     tlmk::pairWordKernel<<<(unsigned)((npairs + 255) / 256), 256, 0, h->stream>>>(
         h->dMat, h->nx, h->ny, h->nz, h->px, tlmk::makeFastDiv((unsigned)(h->px / 2)),
         tlmk::makeFastDiv((unsigned)h->ny), (unsigned)npairs, h->dPairWord);
@@ -882,6 +898,29 @@ tlm_status ensurePair(tlm_solver *h)
     TLM_CU(h, cudaGetLastError());
     h->pair = std::move(plan);
     return TLM_OK;
+}
+
+// The plan is tried once per prepare (and again after reclaim); without one
+// (not enough memory for the second set of stub planes, no tensor maps) the
+// handle keeps stepping one step per launch and holds nothing of it.
+tlm_status ensurePair(tlm_solver *h)
+{
+    if (h->pairTried) return TLM_OK;
+    const size_t before = h->devBytes;
+    const std::string err = h->err;
+    tlm_status st = planPair(h);
+    h->pairBytes = h->devBytes - before;
+    if (!h->pair)
+    {
+        dropPair(h);
+        if (st == TLM_ENOMEM)
+        {
+            st = TLM_OK;
+            h->err = err;
+        }
+    }
+    h->pairTried = true;
+    return st;
 }
 
 // Whether the next two steps may share a pass: FP32 in the default shape,
@@ -1005,6 +1044,7 @@ tlm_status ensureResident(tlm_solver *h)
         devAlloc(h, &h->dEpair, share) != TLM_OK)
     {
         cudaGetLastError();
+        devFree(h, h->dResPack);
         h->resBy = 0;
         return TLM_OK;
     }

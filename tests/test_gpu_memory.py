@@ -1,0 +1,81 @@
+"""A handle gives up the scratch of its two-step passes for memory it cannot do without.
+
+With the card nearly full, reading the state needs more scratch than is left
+beside the plan, and less than is left without it: the state is read all the
+same, later steps run without a plan or with a new one, and everything is
+bitwise what a handle with room gives. Where there is no room for a plan the
+handle steps without one and holds nothing of it. Each case runs in a process of
+its own: the library's memory pool keeps what earlier handles had."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from emsolver_b200.runner import build_solver, records
+from tests.test_gpu_pair import grid
+
+pytestmark = pytest.mark.gpu
+
+NX, NY, NZ = 304, 256, 256
+MIB = 1 << 20
+
+
+def fill(torch, leave):
+    """Device memory taken until `leave` bytes are free."""
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    return torch.empty(free - leave, dtype=torch.uint8, device="cuda")
+
+
+def state_read_beside_a_plan():
+    import torch
+    w = grid(NX, NY, NZ, 0.3, 10, seed=1)
+    nodes = NX * NY * NZ
+    state, plan = 48 * nodes, 18 * nodes
+    out = []
+    for tight in (True, False):
+        s = build_solver(w)
+        s.step(4)
+        assert s.stepsPerPass() == 2
+        hog = fill(torch, state - plan // 2) if tight else None
+        got = [s.pulses(), s.stubs()]
+        s.step(6)
+        del hog
+        torch.cuda.empty_cache()
+        got += [s.pulses(), s.stubs(), records(s, w, f64=True)]
+        s.close()
+        out.append(got)
+    for a, b in zip(out[0][:4], out[1][:4]):
+        assert np.array_equal(a, b)
+    for k in out[0][4]:
+        assert np.array_equal(out[0][4][k], out[1][4][k]), k
+
+
+def no_room_for_a_plan():
+    import torch
+    w = grid(NX, NY, NZ, 0.3, 6, seed=1)
+    s = build_solver(w)
+    s.step(1)                     # a single step: no plan yet
+    before = s.deviceBytes()
+    hog = fill(torch, 300 * MIB)
+    s.step(3)
+    assert s.stepsPerPass() == 1 and s.deviceBytes() == before
+    del hog
+    torch.cuda.empty_cache()
+    got = s.pulses()
+    s.close()
+    r = build_solver(w)
+    r.step(4)
+    assert np.array_equal(got, r.pulses())
+    r.close()
+
+
+@pytest.mark.parametrize("case", ["state_read_beside_a_plan", "no_room_for_a_plan"])
+def test_nearly_full_card(built, case):
+    pytest.importorskip("torch")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", f"from tests import test_gpu_memory as t; t.{case}()"], cwd=root,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]

@@ -989,15 +989,16 @@ __global__ void __launch_bounds__(128) edgeFlagKernel(const unsigned *__restrict
     if (threadIdx.x == 0) flags[blockIdx.x] = other ? 1 : 0;
 }
 
-// A component of extents n in the reference's layout (x fastest, no padding).
-__global__ void __launch_bounds__(256) packFieldKernel(const float *__restrict__ f, Dims d, int n0, int n1, long long total,
-                                                       float *__restrict__ out)
+// `count` values, from the one numbered `first` on, of a component of extents n
+// in the reference's layout (x fastest, no padding).
+__global__ void __launch_bounds__(256) packFieldKernel(const float *__restrict__ f, Dims d, int n0, int n1, long long first,
+                                                       long long count, float *__restrict__ out)
 {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < count;
          t += (long long)gridDim.x * blockDim.x)
     {
-        const int i = (int)(t % n0);
-        const long long r = t / n0;
+        const int i = (int)((first + t) % n0);
+        const long long r = (first + t) / n0;
         out[t] = f[d.at(i, (int)(r % n1), (int)(r / n1))];
     }
 }
@@ -1966,15 +1967,27 @@ tlm_status fdtd_get_field(fdtd_handle h, int which, float *out, size_t cap, size
     if (!out) return TLM_OK;
     if (cap < (size_t)h->len[which]) return h->fail(TLM_EINVAL, "output smaller than the field");
     Guard gd(h->device);
+    // packed in pieces of at most 64 MiB, smaller ones on a card that is full
+    const long long total = h->len[which];
+    long long piece = std::min<long long>(total, 1LL << 24);
     float *packed = nullptr;
-    FD_TRY(alloc(h, &packed, (size_t)h->len[which] * 4));
+    while (alloc(h, &packed, (size_t)piece * 4) != TLM_OK)
+    {
+        if (piece <= 1024) return TLM_ENOMEM;
+        piece /= 2;
+    }
     const int a = which % 3;  // E: one more entry on the axes other than a; H: one more on a
     const int n0 = h->d.nx + ((which < 3) == (a != 0) ? 1 : 0), n1 = h->d.ny + ((which < 3) == (a != 1) ? 1 : 0);
-    fdk::packFieldKernel<<<tlmi::gridBlocksFor(h->len[which]), 256, 0, h->stream>>>(h->field(which), h->d, n0, n1,
-                                                                                  h->len[which], packed);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(out, packed, (size_t)h->len[which] * 4, cudaMemcpyDeviceToHost, h->stream);
+    cudaError_t e = cudaSuccess;
+    for (long long first = 0; first < total && e == cudaSuccess; first += piece)
+    {
+        const long long count = std::min(piece, total - first);
+        fdk::packFieldKernel<<<tlmi::gridBlocksFor(count), 256, 0, h->stream>>>(h->field(which), h->d, n0, n1, first,
+                                                                              count, packed);
+        e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(out + first, packed, (size_t)count * 4, cudaMemcpyDeviceToHost, h->stream);
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     release(h, packed);
     return h->cuda(e, "field read-back");

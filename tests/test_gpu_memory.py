@@ -1,10 +1,11 @@
-"""A handle gives up the scratch of its two-step passes for memory it cannot do without.
+"""Nearly full cards: optional scratch gives way, and what is read back needs little.
 
-With the card nearly full, reading the state needs more scratch than is left
+Two-step passes: with the card nearly full, reading the state needs more scratch than is left
 beside the plan, and less than is left without it: the state is read all the
 same, later steps run without a plan or with a new one, and everything is
 bitwise what a handle with room gives. Where there is no room for a plan the
-handle steps without one and holds nothing of it. Each case runs in a process of
+handle steps without one and holds nothing of it. FDTD fields are read in pieces
+that fit what is left. Each case runs in a process of
 its own: the library's memory pool keeps what earlier handles had."""
 import os
 import subprocess
@@ -72,7 +73,28 @@ def no_room_for_a_plan():
     r.close()
 
 
-@pytest.mark.parametrize("case", ["state_read_beside_a_plan", "no_room_for_a_plan"])
+def field_read_on_a_full_card():
+    import torch
+    from emsolver_b200 import workloads
+    from emsolver_b200.fdtd import FIELDS, build_fdtd
+    small, large = workloads.heterogeneous(n=16, steps=3), workloads.heterogeneous(n=288, steps=3)
+    s = build_fdtd(small)         # loads the kernels
+    s.run()
+    s.fields()
+    s.close()
+    s = build_fdtd(large)
+    s.run()
+    hog = fill(torch, 6 * MIB)
+    got = s.fields()
+    del hog
+    torch.cuda.empty_cache()
+    assert np.abs(got["Ez"]).max() > 0.0
+    for k in FIELDS:              # in one piece or in others
+        assert np.array_equal(got[k], s.field(k)), k
+    s.close()
+
+
+@pytest.mark.parametrize("case", ["field_read_on_a_full_card", "state_read_beside_a_plan", "no_room_for_a_plan"])
 def test_nearly_full_card(built, case):
     pytest.importorskip("torch")
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))

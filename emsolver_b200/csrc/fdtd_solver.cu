@@ -1177,15 +1177,22 @@ void freeMonitors(fdtd_solver *h)
     h->prepared = false;
 }
 
-void freeAll(fdtd_solver *h)
+// The second field buffer and what else only fused passes need.
+void dropFused(fdtd_solver *h)
 {
-    freeMonitors(h);
-    for (int b = 0; b < 2; ++b) release(h, h->dBuf[b]);
-    release(h, h->dCls);
-    release(h, h->dTab);
+    release(h, h->dBuf[1]);
     release(h, h->dFlags);
     release(h, h->dFault);
     h->maps.reset();
+}
+
+void freeAll(fdtd_solver *h)
+{
+    freeMonitors(h);
+    dropFused(h);
+    release(h, h->dBuf[0]);
+    release(h, h->dCls);
+    release(h, h->dTab);
     for (int c = 0; c < 3; ++c)
     {
         release(h, h->dCa[c]);
@@ -1436,6 +1443,26 @@ tlm_status fusedMaps(fdtd_solver *h)
                          "cudaFuncSetAttribute(fusedStepKernel)");
     });
     return st;
+}
+
+// Everything fused passes need beyond the in-place sweeps.
+tlm_status planFused(fdtd_solver *h)
+{
+    const fdk::Dims &d = h->d;
+    const size_t field = 6 * (size_t)h->P * 4;
+    FD_TRY(alloc(h, &h->dBuf[1], field));
+    if (reinterpret_cast<uintptr_t>(h->dBuf[1]) & 15) return h->fail(TLM_ECUDA, "field allocation not 16-byte aligned");
+    FD_CU(h, cudaMemsetAsync(h->dBuf[1], 0, field, h->stream));
+    int sms = 0;
+    FD_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    chooseFused(h, sms);
+    FD_TRY(alloc(h, &h->dFault, sizeof(unsigned)));
+    FD_CU(h, cudaMemsetAsync(h->dFault, 0, sizeof(unsigned), h->stream));
+    FD_TRY(fusedMaps(h));
+    const size_t nf = (size_t)h->ntx * h->nty * (d.nz + 1);
+    FD_TRY(alloc(h, &h->dFlags, nf));
+    fdk::edgeFlagKernel<<<(unsigned)nf, 128, 0, h->stream>>>(h->dCls, d, h->TX, h->TY, h->ntx, h->dFlags);
+    return h->cuda(cudaGetLastError(), "edge flags");
 }
 
 // more: another step follows at once (its sources may go in with this step's tail)
@@ -1739,13 +1766,10 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     // within a plane are 32-bit); no_staging asks for the in-place sweeps
     const bool fused = need + field + spare <= avail && !cfg->no_staging && (long long)d.px * (ny + 1) < (1LL << 30) &&
                        tlmi::tensorMapEncoder() != nullptr;
-    for (int b = 0; b < (fused ? 2 : 1); ++b)
-    {
-        FD_TRY(alloc(h, &h->dBuf[b], field));
-        if (reinterpret_cast<uintptr_t>(h->dBuf[b]) & 15)  // vector loads
-            return h->fail(TLM_ECUDA, "field allocation not 16-byte aligned");
-        FD_CU(h, cudaMemsetAsync(h->dBuf[b], 0, field, h->stream));
-    }
+    FD_TRY(alloc(h, &h->dBuf[0], field));
+    if (reinterpret_cast<uintptr_t>(h->dBuf[0]) & 15)  // vector loads
+        return h->fail(TLM_ECUDA, "field allocation not 16-byte aligned");
+    FD_CU(h, cudaMemsetAsync(h->dBuf[0], 0, field, h->stream));
     FD_TRY(alloc(h, &h->dCls, classes));
     FD_CU(h, cudaMemsetAsync(h->dCls, 0, classes, h->stream));
     if (h->haveDiel)
@@ -1800,19 +1824,6 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
         release(h, dProps);
         FD_TRY(st);
     }
-    if (fused)
-    {
-        int sms = 0;
-        FD_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-        chooseFused(h, sms);
-        FD_TRY(alloc(h, &h->dFault, sizeof(unsigned)));
-        FD_CU(h, cudaMemsetAsync(h->dFault, 0, sizeof(unsigned), h->stream));
-        FD_TRY(fusedMaps(h));
-        const size_t nf = (size_t)h->ntx * h->nty * (nz + 1);
-        FD_TRY(alloc(h, &h->dFlags, nf));
-        fdk::edgeFlagKernel<<<(unsigned)nf, 128, 0, h->stream>>>(h->dCls, d, h->TX, h->TY, h->ntx, h->dFlags);
-        FD_CU(h, cudaGetLastError());
-    }
     // Mur planes: x faces (Ey, Ez), y faces (Ex, Ez), z faces (Ex, Ey)
     const int n1[6] = { ny, ny + 1, nx, nx + 1, nx, nx + 1 };
     const int n2[6] = { nz + 1, nz, nz + 1, nz, ny + 1, ny };
@@ -1827,6 +1838,17 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     h->mur.cMur = h->cMur;
     FD_TRY(alloc(h, &h->mur.snap, (size_t)total * 4));
     FD_CU(h, cudaMemsetAsync(h->mur.snap, 0, (size_t)total * 4, h->stream));
+    if (fused)
+    {
+        // last, and without what another handle took in the meantime the
+        // sweeps run in place
+        const std::string err = h->err;
+        if (planFused(h) != TLM_OK)
+        {
+            dropFused(h);
+            h->err = err;
+        }
+    }
     FD_CU(h, cudaStreamSynchronize(h->stream));
     h->planeSources.clear();
     h->ports.clear();

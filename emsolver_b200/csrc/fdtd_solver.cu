@@ -1037,6 +1037,9 @@ struct fdtd_solver
     int layout = 0, TX = 0, TY = 0, ntx = 0, nty = 0, nchunk = 0;
     fdk::Mur mur{};
     float *field(int c) const { return dBuf[cur] + c * P; }
+    tlmi::Lender lender;    // the second field buffer
+    bool planning = false;  // allocating it
+    bool lent = false;      // given back since set-up
     // sources
     struct Src
     {
@@ -1132,7 +1135,7 @@ struct Guard
 template <class T> tlm_status alloc(fdtd_solver *h, T **p, size_t bytes)
 {
     void *q = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&q, std::max<size_t>(bytes, 1), h->pool, h->stream);
+    cudaError_t e = tlmi::poolAlloc(h->device, h->pool, h->stream, h->planning, &q, std::max<size_t>(bytes, 1));
     if (e != cudaSuccess)
     {
         cudaGetLastError();
@@ -1445,11 +1448,30 @@ tlm_status fusedMaps(fdtd_solver *h)
     return st;
 }
 
+// For reclaim: the state moves to the first buffer's place, and the sweeps run
+// in place from now on (or until there is room again).
+bool giveBufferBack(fdtd_solver *h)
+{
+    if (!h->dBuf[1]) return false;
+    if (h->cur == 1) std::swap(h->dBuf[0], h->dBuf[1]);
+    h->cur = 0;
+    dropFused(h);
+    h->lent = true;
+    cudaStreamSynchronize(h->stream);
+    return true;
+}
+
+size_t fieldBytes(const fdtd_solver *h) { return 6 * (size_t)h->P * 4; }
+bool roomForFused(const fdtd_solver *h)
+{
+    return fieldBytes(h) + ((size_t)256 << 20) <= tlmi::poolAvailable(h->device);
+}
+
 // Everything fused passes need beyond the in-place sweeps.
-tlm_status planFused(fdtd_solver *h)
+tlm_status allocFused(fdtd_solver *h)
 {
     const fdk::Dims &d = h->d;
-    const size_t field = 6 * (size_t)h->P * 4;
+    const size_t field = fieldBytes(h);
     FD_TRY(alloc(h, &h->dBuf[1], field));
     if (reinterpret_cast<uintptr_t>(h->dBuf[1]) & 15) return h->fail(TLM_ECUDA, "field allocation not 16-byte aligned");
     FD_CU(h, cudaMemsetAsync(h->dBuf[1], 0, field, h->stream));
@@ -1463,6 +1485,17 @@ tlm_status planFused(fdtd_solver *h)
     FD_TRY(alloc(h, &h->dFlags, nf));
     fdk::edgeFlagKernel<<<(unsigned)nf, 128, 0, h->stream>>>(h->dCls, d, h->TX, h->TY, h->ntx, h->dFlags);
     return h->cuda(cudaGetLastError(), "edge flags");
+}
+void planFused(fdtd_solver *h)
+{
+    const std::string err = h->err;
+    h->planning = true;
+    if (allocFused(h) != TLM_OK)
+    {
+        dropFused(h);
+        h->err = err;
+    }
+    h->planning = false;
 }
 
 // more: another step follows at once (its sources may go in with this step's tail)
@@ -1690,6 +1723,7 @@ tlm_status fdtd_create(fdtd_handle *out, int device)
         g_fdtdErr = "memory pool unavailable";
         return TLM_ECUDA;
     }
+    tlmi::enlist(h->lender, device, [h] { return giveBufferBack(h); });
     *out = h;
     return TLM_OK;
 }
@@ -1699,6 +1733,7 @@ tlm_status fdtd_destroy(fdtd_handle h)
     if (!h) return TLM_OK;
     {
         Guard g(h->device);
+        tlmi::delist(h->lender);
         cudaStreamSynchronize(h->stream);
         freeAll(h);
         cudaStreamSynchronize(h->stream);
@@ -1735,9 +1770,11 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     if (cfg->waveform < 0 || cfg->waveform > TLM_WAVE_TABLE) return h->fail(TLM_EINVAL, "unknown waveform");
     if (cfg->record_every < 0 || cfg->huy_offset < 0) return h->fail(TLM_EINVAL, "negative record_every or huy_offset");
     Guard gd(h->device);
+    std::lock_guard<std::recursive_timed_mutex> lk(h->lender.busy);
     cudaStreamSynchronize(h->stream);
     freeAll(h);
     h->configured = false;
+    h->lent = false;
     h->g = *grid;
     h->cfg = *cfg;
     h->mat.swap(hostMat);
@@ -1758,9 +1795,10 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     h->len[5] = (long long)nx * ny * (nz + 1);
     h->P = (long long)d.px * (ny + 1) * (nz + 1);
     h->cur = 0;
-    const size_t field = 6 * (size_t)h->P * 4, classes = (size_t)h->P * 4, mixed = h->haveDiel ? 6 * (size_t)h->P * 4 : 0;
+    const size_t field = fieldBytes(h), classes = (size_t)h->P * 4, mixed = h->haveDiel ? 6 * (size_t)h->P * 4 : 0;
     const size_t need = field + classes + mixed, spare = (size_t)256 << 20;
-    const size_t avail = tlmi::poolAvailable(h->device);
+    size_t avail = tlmi::poolAvailable(h->device);
+    if (need + spare > avail && tlmi::reclaim(h->device)) avail = tlmi::poolAvailable(h->device);
     if (need + spare > avail) return h->fail(TLM_ENOMEM, "grid needs " + std::to_string(need >> 20) + " MiB of HBM");
     // a second field buffer for fused passes where it fits (their lane offsets
     // within a plane are 32-bit); no_staging asks for the in-place sweeps
@@ -1838,17 +1876,7 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     h->mur.cMur = h->cMur;
     FD_TRY(alloc(h, &h->mur.snap, (size_t)total * 4));
     FD_CU(h, cudaMemsetAsync(h->mur.snap, 0, (size_t)total * 4, h->stream));
-    if (fused)
-    {
-        // last, and without what another handle took in the meantime the
-        // sweeps run in place
-        const std::string err = h->err;
-        if (planFused(h) != TLM_OK)
-        {
-            dropFused(h);
-            h->err = err;
-        }
-    }
+    if (fused) planFused(h);
     FD_CU(h, cudaStreamSynchronize(h->stream));
     h->planeSources.clear();
     h->ports.clear();
@@ -1939,8 +1967,12 @@ tlm_status fdtd_step(fdtd_handle h, int n_steps)
     FD_TRY(ready(h));
     if (n_steps < 0) return h->fail(TLM_EINVAL, "n_steps must be >= 0");
     Guard gd(h->device);
+    std::lock_guard<std::recursive_timed_mutex> lk(h->lender.busy);
     FD_TRY(prepare(h));
     FD_TRY(ensureRecords(h, (long long)h->curStep + n_steps));
+    // (looking for room takes as long as a few steps)
+    if (h->lent && n_steps >= 64 && roomForFused(h)) planFused(h);
+    if (h->dBuf[1]) h->lent = false;
     for (int t = 0; t < n_steps; ++t)
     {
         FD_TRY(launchStep(h, h->curStep, t + 1 < n_steps));
@@ -1989,6 +2021,7 @@ tlm_status fdtd_get_field(fdtd_handle h, int which, float *out, size_t cap, size
     if (!out) return TLM_OK;
     if (cap < (size_t)h->len[which]) return h->fail(TLM_EINVAL, "output smaller than the field");
     Guard gd(h->device);
+    std::lock_guard<std::recursive_timed_mutex> lk(h->lender.busy);
     // packed in pieces of at most 64 MiB, smaller ones on a card that is full
     const long long total = h->len[which];
     long long piece = std::min<long long>(total, 1LL << 24);

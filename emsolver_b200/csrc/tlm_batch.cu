@@ -197,7 +197,7 @@ template <class S> MemberDesc<S> makeDesc(tlm_solver *h)
 cudaError_t batchAlloc(tlm_batch_s *b, void **p, size_t bytes)
 {
     cudaMemPool_t pool = devicePool(b->device);
-    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, b->stream) : cudaMallocAsync(p, bytes, b->stream);
+    return pool ? tlmi::poolAlloc(b->device, pool, b->stream, false, p, bytes) : cudaMallocAsync(p, bytes, b->stream);
 }
 void batchFree(tlm_batch_s *b, void *p)
 {

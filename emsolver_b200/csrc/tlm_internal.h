@@ -9,7 +9,9 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <functional>
 #include <memory>
+#include <mutex>
 #include <type_traits>
 #include <string>
 #include <vector>
@@ -194,6 +196,22 @@ struct PairPlan;
 // two are even, at 88^3 14.2 against 13.3 us).
 constexpr long long kPairMinNodes = 1LL << 20;
 inline bool pairStorage(int storage, long long P) { return storage == TLM_STORE_F32 && P >= kPairMinNodes; }
+
+// A handle's share in the device memory that handles hold for speed alone and
+// give back when another allocation finds no room: the plan of two-step passes,
+// the second field buffer of the FDTD solver. The handle holds `busy` while it
+// uses that memory.
+struct Lender
+{
+    int device = -1;
+    std::recursive_timed_mutex busy;
+    std::function<bool()> giveBack;  // called with `busy` held; true if there was anything
+};
+void enlist(Lender &l, int device, std::function<bool()> giveBack);
+void delist(Lender &l);
+// Take back what the device's handles can do without, but for those that have
+// been at work for milliseconds; true if there was anything.
+bool reclaim(int device);
 } // namespace tlmi
 
 struct tlm_solver
@@ -294,6 +312,8 @@ struct tlm_solver
     std::shared_ptr<tlmi::PairPlan> pair;
     bool pairTried = false;
     size_t pairBytes = 0;                // device bytes of the plan
+    bool planning = false;               // allocating for it
+    tlmi::Lender lender;
     unsigned *dPairFlags = nullptr;
     unsigned *dPairWord = nullptr;       // material word of every node pair
     int *dSpecRow = nullptr;             // first entry of dSpec in every row of nodes
@@ -360,16 +380,15 @@ namespace tlmi {
 // Device memory of a handle comes from a per-device stream-ordered pool that
 // keeps freed blocks for reuse (no device-wide synchronisation and no
 // driver round trip per allocation), ordered on the handle's stream.
-// What a handle can do without (the plan of two-step passes) is given up for
-// what it cannot: true if there was anything.
-bool reclaim(tlm_solver *h);
-inline cudaError_t poolAlloc(tlm_solver *h, void **q, size_t bytes)
+// From the device's pool; where that has no room, other scratch of the device
+// gives way unless `optional` (reclaim).
+inline cudaError_t poolAlloc(int device, cudaMemPool_t pool, cudaStream_t stream, bool optional, void **q, size_t bytes)
 {
-    cudaError_t e = cudaMallocFromPoolAsync(q, bytes, h->pool, h->stream);
-    if (e == cudaErrorMemoryAllocation && reclaim(h))
+    cudaError_t e = cudaMallocFromPoolAsync(q, bytes, pool, stream);
+    if (e == cudaErrorMemoryAllocation && !optional && reclaim(device))
     {
         cudaGetLastError();
-        e = cudaMallocFromPoolAsync(q, bytes, h->pool, h->stream);
+        e = cudaMallocFromPoolAsync(q, bytes, pool, stream);
     }
     return e;
 }
@@ -378,7 +397,7 @@ template <class T> tlm_status devAlloc(tlm_solver *h, T **p, size_t bytes)
     *p = nullptr;
     if (bytes == 0) return TLM_OK;
     void *q = nullptr;
-    cudaError_t e = poolAlloc(h, &q, bytes);
+    cudaError_t e = poolAlloc(h->device, h->pool, h->stream, h->planning, &q, bytes);
     if (e != cudaSuccess)
     {
         cudaGetLastError();
@@ -393,7 +412,7 @@ template <class T> tlm_status devAlloc(tlm_solver *h, T **p, size_t bytes)
 template <class T> tlm_status tmpAlloc(tlm_solver *h, T **p, size_t bytes)
 {
     void *q = nullptr;
-    cudaError_t e = poolAlloc(h, &q, bytes > 0 ? bytes : 1);
+    cudaError_t e = poolAlloc(h->device, h->pool, h->stream, h->planning, &q, bytes > 0 ? bytes : 1);
     if (e != cudaSuccess)
     {
         cudaGetLastError();

@@ -13,6 +13,7 @@
 #include "tlm_step_kernel.cuh"
 
 #include <algorithm>
+#include <chrono>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -59,10 +60,45 @@ namespace tlmi {
 
 
 
+namespace {
+std::mutex g_lendersMutex;
+std::vector<Lender *> g_lenders;
+} // namespace
+
+void enlist(Lender &l, int device, std::function<bool()> giveBack)
+{
+    l.device = device;
+    l.giveBack = std::move(giveBack);
+    std::lock_guard<std::mutex> lk(g_lendersMutex);
+    g_lenders.push_back(&l);
+}
+
+void delist(Lender &l)
+{
+    std::lock_guard<std::mutex> lk(g_lendersMutex);
+    g_lenders.erase(std::remove(g_lenders.begin(), g_lenders.end(), &l), g_lenders.end());
+}
+
+// (a handle that waits here holds its own `busy` and the list's mutex, of which
+// the former is only ever tried, so no two wait for each other)
+bool reclaim(int device)
+{
+    bool any = false;
+    std::lock_guard<std::mutex> lk(g_lendersMutex);
+    for (Lender *l : g_lenders)
+    {
+        if (l->device != device || !l->busy.try_lock_for(std::chrono::milliseconds(5))) continue;
+        any = l->giveBack() || any;
+        l->busy.unlock();
+    }
+    return any;
+}
+
 // Forget the plan of two-step passes (or what a failed attempt at one has
 // allocated so far) with its memory; the next step may plan again.
 void dropPair(tlm_solver *h)
 {
+    std::lock_guard<std::recursive_timed_mutex> lk(h->lender.busy);
     h->pair.reset();
     h->pairTried = false;
     devFree(h, h->dPairFlags);
@@ -70,17 +106,15 @@ void dropPair(tlm_solver *h)
     devFree(h, h->dSpecRow);
     devFree(h, h->dStubAlt);
     devFree(h, h->dEpair);
-    h->devBytes -= h->pairBytes;
     h->pairBytes = 0;
 }
 
-bool reclaim(tlm_solver *h)
+// For reclaim.
+bool givePairBack(tlm_solver *h)
 {
     if (!h->pair) return false;
     dropPair(h);
-    // the blocks go back to the device: the pool does not join them into a larger one
     cudaStreamSynchronize(h->stream);
-    cudaMemPoolTrimTo(h->pool, 0);
     return true;
 }
 
@@ -908,8 +942,11 @@ tlm_status ensurePair(tlm_solver *h)
     if (h->pairTried) return TLM_OK;
     const size_t before = h->devBytes;
     const std::string err = h->err;
+    h->planning = true;
     tlm_status st = planPair(h);
+    h->planning = false;
     h->pairBytes = h->devBytes - before;
+    h->devBytes = before;
     if (!h->pair)
     {
         dropPair(h);
@@ -1180,6 +1217,7 @@ template <class R> tlm_status launchEpilogue(tlm_solver *h, long long base, int 
 tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stopped)
 {
     if (stopped) *stopped = false;
+    std::lock_guard<std::recursive_timed_mutex> lk(h->lender.busy);
     TLM_TRY(prepare(h));
     int remaining = nsteps;
     while (remaining > 0)
@@ -1627,6 +1665,7 @@ tlm_status tlm_create(tlm_handle *out, int device)
         delete h;
         return TLM_ENOMEM;
     }
+    enlist(h->lender, device, [h] { return givePairBack(h); });
     *out = h;
     return TLM_OK;
 }
@@ -1637,6 +1676,7 @@ tlm_status tlm_destroy(tlm_handle h)
     if (busy(h)) return h->fail(TLM_EBUSY, "cannot destroy a running handle");
     if (h->batch) return h->fail(TLM_EBUSY, "detach the handle from its batch first");
     DeviceGuard dg(h->device);
+    delist(h->lender);
     cudaStreamSynchronize(h->stream);
     freeAll(h);
     if (h->dElatest) cudaFreeAsync(h->dElatest, h->stream);
@@ -1793,8 +1833,10 @@ tlm_status tlm_setup(tlm_handle h, const tlm_grid *grid, const uint8_t *mat, siz
     // taken and the device query, a few hundred microseconds, is skipped)
     if (!poolCovers(h->device, need))
     {
-        const size_t freeB = poolAvailable(h->device);
-        if (need + (size_t)(256u << 20) > freeB)
+        const size_t spare = (size_t)(256u << 20);
+        size_t freeB = poolAvailable(h->device);
+        if (need + spare > freeB && reclaim(h->device)) freeB = poolAvailable(h->device);
+        if (need + spare > freeB)
             return h->fail(TLM_ENOMEM, "grid needs " + std::to_string(need >> 20) + " MiB of HBM, " +
                                            std::to_string(freeB >> 20) + " MiB free");
     }
@@ -2653,7 +2695,7 @@ tlm_status tlm_get_stream(tlm_handle h, void **stream)
 tlm_status tlm_device_bytes(tlm_handle h, size_t *bytes)
 {
     TLM_TRY(checkHandle(h));
-    if (bytes) *bytes = h->devBytes;
+    if (bytes) *bytes = h->devBytes + h->pairBytes;
     return TLM_OK;
 }
 
@@ -2692,6 +2734,7 @@ tlm_status tlm_steps_per_pass(tlm_handle h, int *steps)
     TLM_TRY(checkReady(h));
     if (!steps) return h->fail(TLM_EINVAL, "null output");
     DeviceGuard dg(h->device);
+    std::lock_guard<std::recursive_timed_mutex> lk(h->lender.busy);
     TLM_TRY(prepare(h));
     *steps = 1;
     if (residentAllowed(h))

@@ -5,7 +5,8 @@ beside the plan, and less than is left without it: the state is read all the
 same, later steps run without a plan or with a new one, and everything is
 bitwise what a handle with room gives. Where there is no room for a plan the
 handle steps without one and holds nothing of it. FDTD fields are read in pieces
-that fit what is left. Each case runs in a process of
+that fit what is left. A further handle takes back what others hold for speed alone (plans, second
+field buffers). Each case runs in a process of
 its own: the library's memory pool keeps what earlier handles had."""
 import os
 import subprocess
@@ -94,7 +95,57 @@ def field_read_on_a_full_card():
     s.close()
 
 
-@pytest.mark.parametrize("case", ["field_read_on_a_full_card", "state_read_beside_a_plan", "no_room_for_a_plan"])
+def second_handle_beside_a_plan():
+    import torch
+    nodes = NX * NY * NZ
+    need, plan = (96 + 12 + 1) * nodes, 18 * nodes
+    w = grid(NX, NY, NZ, 0.3, 6, seed=1)
+    a = build_solver(w)
+    a.step(3)
+    assert a.stepsPerPass() == 2
+    hog = fill(torch, need + 256 * MIB - plan // 2)
+    b = build_solver(w)           # takes the plan's memory
+    b.step(3)
+    a.step(3)
+    b.step(3)
+    del hog                       # (reading the state needs 48 B per node)
+    torch.cuda.empty_cache()
+    got = [(s.pulses(), s.stubs()) for s in (a, b)]
+    b.close()
+    b = build_solver(w)
+    b.step(6)
+    for p, v in got:
+        assert np.array_equal(p, b.pulses()) and np.array_equal(v, b.stubs())
+
+
+def several_fdtd_handles():
+    import torch
+    from emsolver_b200 import workloads
+    from emsolver_b200.fdtd import FIELDS, build_fdtd
+    w = workloads.heterogeneous(n=320, steps=70)
+    plane = 4 * 324 * 321 * 321
+    build_fdtd(workloads.heterogeneous(n=16, steps=3)).run()
+    hog = fill(torch, 4 * 13 * plane + 600 * MIB)
+    s = [build_fdtd(w) for _ in range(4)]    # 13 planes each, the first two with six more until others need them
+    for q in s:
+        q.step(3)
+    s.pop(0).close()
+    s.pop(0).close()
+    for q in s:                              # with room again
+        q.step(67)
+    got = [q.fields() for q in s]
+    del hog, s
+    torch.cuda.empty_cache()
+    r = build_fdtd(w)
+    r.run()
+    want = r.fields()
+    assert np.abs(want["Ez"]).max() > 0.0
+    for g in got:
+        for k in FIELDS:
+            assert np.array_equal(g[k], want[k]), k
+
+
+@pytest.mark.parametrize("case", ["second_handle_beside_a_plan", "several_fdtd_handles", "field_read_on_a_full_card", "state_read_beside_a_plan", "no_room_for_a_plan"])
 def test_nearly_full_card(built, case):
     pytest.importorskip("torch")
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))

@@ -313,6 +313,7 @@ struct tlm_solver
     bool pairTried = false;
     size_t pairBytes = 0;                // device bytes of the plan
     bool planning = false;               // allocating for it
+    bool noPair = false;                 // the server's budget has no room for it
     tlmi::Lender lender;
     unsigned *dPairFlags = nullptr;
     unsigned *dPairWord = nullptr;       // material word of every node pair

@@ -51,7 +51,9 @@ struct Request
     std::vector<PortSpec> ports;
     std::vector<int> probes;  // i j k per probe
     std::vector<double> freqs;
-    size_t footprint = 0;
+    size_t footprint = 0;     // device bytes it needs
+    size_t held = 0;          // device bytes counted for it while it runs
+    bool planned = false;     // with a plan of two-step passes among them
     long long nodes = 0;      // padded cells of the grid
     double work = 0.0;        // nodes x total_steps
     bool solo = false;        // stepped on its own stream by the single-grid kernels, not in the batch
@@ -131,10 +133,7 @@ size_t footprintOf(const tlm_grid &g, const std::vector<uint8_t> &mat, const tlm
             break;
         }
     const size_t steps = (size_t)std::max(cfg.total_steps, 1);
-    // (large FP32 grids step two steps per pass, with a second set of stubs and
-    // every node pair's energy share and material word)
-    const bool pair = tlmi::pairStorage(cfg.storage, (long long)P);
-    return 2 * 12 * P * sb + (diel ? (pair ? 2 : 1) * 3 * P * rb : 0) + (pair ? 6 * P : 0) + P + steps * (nports * 2 + nprobes * 3 + 1) * 8 +
+    return 2 * 12 * P * sb + (diel ? 3 * P * rb : 0) + P + steps * (nports * 2 + nprobes * 3 + 1) * 8 +
            nports * nfreq * 32 + steps * rb + (1u << 20);
 }
 
@@ -175,6 +174,7 @@ tlm_status startRequest(tlm_server_s *s, Request &r)
         r.error = tlm_last_error(nullptr);
         return st;
     }
+    r.h->noPair = !r.planned;
     auto bad = [&](tlm_status e) {
         r.error = tlm_last_error(r.h);
         tlm_destroy(r.h);
@@ -265,7 +265,7 @@ void retire(tlm_server_s *s, std::unique_lock<std::mutex> &lk)
         }
         lk.lock();
         r->finished = Clock::now();
-        s->used -= r->footprint;
+        s->used -= r->held;
         if (done && r->state != TLM_REQ_CANCELLED)
         {
             r->state = TLM_REQ_DONE;
@@ -313,8 +313,15 @@ void workerMain(tlm_server_s *s)
             plannedNodes += r->nodes;
             r->state = TLM_REQ_RUNNING;
             r->started = Clock::now();
-            planned += r->footprint;
-            s->used += r->footprint;
+            // a request of its own stream steps two steps per pass if the budget
+            // has room for that as well (a second set of stubs, every node
+            // pair's energy share and material word)
+            r->solo = s->soloNodes > 0 && r->nodes >= s->soloNodes;
+            const size_t plan = r->solo && tlmi::pairStorage(r->cfg.storage, r->nodes) ? 18 * (size_t)r->nodes : 0;
+            r->planned = planned + r->footprint + plan <= s->budget;
+            r->held = r->footprint + (r->planned ? plan : 0);
+            planned += r->held;
+            s->used += r->held;
             picked.push_back(r);
         }
         if (s->stop)
@@ -322,7 +329,7 @@ void workerMain(tlm_server_s *s)
             for (auto &r : picked)
             {
                 r->state = TLM_REQ_CANCELLED;
-                s->used -= r->footprint;
+                s->used -= r->held;
             }
             break;
         }
@@ -395,7 +402,7 @@ void workerMain(tlm_server_s *s)
                 tlm_destroy(r->h);
                 r->h = nullptr;
                 ++s->failed;
-                s->used -= r->footprint;
+                s->used -= r->held;
             }
             s->running.clear();
         }
@@ -414,11 +421,10 @@ void workerMain(tlm_server_s *s)
             {
                 tlm_destroy(r.h);
                 r.h = nullptr;
-                s->used -= r.footprint;
+                s->used -= r.held;
                 r.finished = Clock::now();
                 continue;
             }
-            r.solo = s->soloNodes > 0 && r.nodes >= s->soloNodes;
             if (ps == TLM_OK && !r.solo && (ps = tlm_batch_attach(s->batch, r.h)) != TLM_OK)
             {
                 r.error = tlm_last_error(nullptr);
@@ -431,7 +437,7 @@ void workerMain(tlm_server_s *s)
                 // request once a running one has freed its memory
                 r.state = TLM_REQ_QUEUED;
                 r.error.clear();
-                s->used -= r.footprint;
+                s->used -= r.held;
                 s->queue.push_front(picked[k]);
                 continue;
             }
@@ -439,7 +445,7 @@ void workerMain(tlm_server_s *s)
             {
                 r.state = TLM_REQ_FAILED;
                 r.finished = Clock::now();
-                s->used -= r.footprint;
+                s->used -= r.held;
                 ++s->failed;
                 continue;
             }

@@ -965,7 +965,7 @@ tlm_status ensurePair(tlm_solver *h)
 // step (slabs), reflected input.
 bool pairAllowed(const tlm_solver *h)
 {
-    return pairStorage(h->storage, h->P) && h->variant == 0 && !h->cfg.no_staging && !h->cfg.general_tiles &&
+    return pairStorage(h->storage, h->P) && !h->noPair && h->variant == 0 && !h->cfg.no_staging && !h->cfg.general_tiles &&
            !h->ghostLo && !h->ghostHi && !surfaceActive(h) && !h->stateIncident;
 }
 

@@ -22,7 +22,7 @@
 //   * one barrier of the block ends a step.
 // The blocks wait on one another, so the launch is cooperative (all blocks
 // resident); every wait is bounded by the global timer, and one that runs out
-// sets kStageTimeout in *fault and stops waiting.
+// sets kResidentTimeout in *fault and stops waiting.
 //
 // The arithmetic of a node is that of the interior and general tile bodies in
 // their order: pulses, stubs and samples are bitwise the same. Energy steps
@@ -35,6 +35,7 @@
 namespace tlmk {
 
 constexpr int kResidentThreads = 512;
+constexpr unsigned kResidentTimeout = 1u << 30;
 constexpr int kResidentSteps = 64;      // steps per launch at most
 constexpr int kResidentEntries = 64;    // source and monitor entries of a brick kept in shared memory
 
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentKernel(const __gr
                         if (t - t0 > kStageWaitNs)
                         {
                             ok = false;
-                            atomicOr(a.fault, kStageTimeout);
+                            atomicOr(a.fault, kResidentTimeout);
                         }
                     }
                 }

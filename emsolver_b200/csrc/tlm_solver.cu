@@ -1090,9 +1090,11 @@ tlm_status ensureResident(tlm_solver *h)
     return TLM_OK;
 }
 
+// (a stage wait limit asks for the staged kernel, see stagedStep)
 bool residentAllowed(const tlm_solver *h)
 {
     return h->storage == TLM_STORE_F32 && h->variant == 0 && !h->cfg.no_staging && !h->cfg.general_tiles &&
+           h->cfg.stage_wait_us == 0 &&
            !h->ghostLo && !h->ghostHi && !surfaceActive(h) && !h->stateIncident &&
            (!h->resTried || h->resBy > 0);
 }
@@ -1294,6 +1296,7 @@ tlm_status syncState(tlm_solver *h)
         unsigned f = 0;
         TLM_CU(h, cudaMemcpy(&f, h->dFault, sizeof(unsigned), cudaMemcpyDeviceToHost));
         if (f & tlmk::kStageTimeout) return h->fail(TLM_ECUDA, "a staged tile's bulk copies never arrived");
+        if (f & tlmk::kResidentTimeout) return h->fail(TLM_ECUDA, "a neighbouring brick's pulses never arrived");
         if (f) return h->fail(TLM_ECUDA, "bounds check tripped, code mask " + std::to_string(f));
     }
     h->doneStep.store(h->curStep);

@@ -128,7 +128,9 @@ typedef struct tlm_config {
                             step fails with TLM_ECUDA; 0 = default (about 2 s),
                             < 0 = at the first poll that finds the stage not
                             ready (exercises the error path). The producer
-                            always lets the copies it issued land */
+                            always lets the copies it issued land. FP32 grids
+                            below 2^20 nodes step with staged tiles only where
+                            this is not 0; passes of two steps keep to it too */
     int near_field;      /* FP16/BF16 storage: radius r in cells of the
                             near-field box, the bounding box of the PEC cells
                             and port cells grown by r (0 = none). Box cells

@@ -36,6 +36,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -682,7 +683,7 @@ template <class L> __global__ void __launch_bounds__(L::kThreads, L::kMinBlocks)
         if (waitOk && !tlmk::mbarWaitBounded(full0 + 8 * sCur, phase))
         {
             waitOk = false;
-            atomicOr(a.fault, tlmk::kStageTimeout);
+            *reinterpret_cast<volatile unsigned *>(a.fault) = tlmk::kStageTimeout;
         }
     };
     wait();
@@ -1032,7 +1033,7 @@ struct fdtd_solver
     float2 *dTab = nullptr;      // their coefficients
     float *dCa[3] = {}, *dCb[3] = {};  // of mixed edges
     unsigned char *dFlags = nullptr;   // [column][plane] of the fused pass
-    unsigned *dFault = nullptr;        // a bulk copy's wait ran out
+    unsigned *fault = nullptr;         // a bulk copy's wait ran out (a FaultWord)
     std::unique_ptr<FdtdMaps> maps;    // boxes of the fused pass in either buffer
     int layout = 0, TX = 0, TY = 0, ntx = 0, nty = 0, nchunk = 0;
     fdk::Mur mur{};
@@ -1180,12 +1181,62 @@ void freeMonitors(fdtd_solver *h)
     h->prepared = false;
 }
 
+// Words of pinned host memory that kernels report a fault in: the host reads one
+// after the synchronisation that ends fdtd_step, where a copy of a device word
+// cost 10 us per call. A page of them is allocated once for all devices and
+// kept; handles beyond its words (null) step in place.
+class FaultWords
+{
+  public:
+    unsigned *take()
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (!page_ && !tried_)
+        {
+            tried_ = true;
+            void *p = nullptr;
+            if (cudaHostAlloc(&p, kWords * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+                cudaGetLastError();
+            page_ = static_cast<unsigned *>(p);
+            if (page_)
+                for (int w = 0; w < kWords; ++w) free_.push_back(page_ + w);
+        }
+        if (free_.empty()) return nullptr;
+        unsigned *w = free_.back();
+        free_.pop_back();
+        *w = 0;
+        return w;
+    }
+    void give(unsigned *w)
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        free_.push_back(w);
+    }
+
+  private:
+    static constexpr int kWords = 4096;
+    std::mutex mu_;
+    bool tried_ = false;
+    unsigned *page_ = nullptr;
+    std::vector<unsigned *> free_;
+};
+FaultWords &faultWords()
+{
+    static FaultWords *words = new FaultWords;  // (handles may outlive static objects)
+    return *words;
+}
+
 // The second field buffer and what else only fused passes need.
 void dropFused(fdtd_solver *h)
 {
     release(h, h->dBuf[1]);
     release(h, h->dFlags);
-    release(h, h->dFault);
+    if (h->fault)
+    {
+        cudaStreamSynchronize(h->stream);  // no kernel writes to it any more
+        faultWords().give(h->fault);
+    }
+    h->fault = nullptr;
     h->maps.reset();
 }
 
@@ -1478,8 +1529,8 @@ tlm_status allocFused(fdtd_solver *h)
     int sms = 0;
     FD_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
     chooseFused(h, sms);
-    FD_TRY(alloc(h, &h->dFault, sizeof(unsigned)));
-    FD_CU(h, cudaMemsetAsync(h->dFault, 0, sizeof(unsigned), h->stream));
+    h->fault = faultWords().take();
+    if (!h->fault) return h->fail(TLM_ENOMEM, "no fault word");
     FD_TRY(fusedMaps(h));
     const size_t nf = (size_t)h->ntx * h->nty * (d.nz + 1);
     FD_TRY(alloc(h, &h->dFlags, nf));
@@ -1605,7 +1656,7 @@ tlm_status launchStep(fdtd_solver *h, int n, bool more)
         fa.mapExy = h->maps->map[h->cur][0];
         fa.mapEz = h->maps->map[h->cur][1];
         fa.mapH = h->maps->map[h->cur][2];
-        fa.fault = h->dFault;
+        fa.fault = h->fault;
         fa.out = h->dBuf[h->cur ^ 1];
         fa.P = h->P;
         fa.d = d;
@@ -1978,11 +2029,8 @@ tlm_status fdtd_step(fdtd_handle h, int n_steps)
         FD_TRY(launchStep(h, h->curStep, t + 1 < n_steps));
         ++h->curStep;
     }
-    unsigned fault = 0;
-    if (h->dFault)
-        FD_CU(h, cudaMemcpyAsync(&fault, h->dFault, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
     FD_CU(h, cudaStreamSynchronize(h->stream));
-    if (fault) return h->fail(TLM_ECUDA, "a field plane's bulk copies never arrived");
+    if (h->fault && *static_cast<volatile unsigned *>(h->fault)) return h->fail(TLM_ECUDA, "a field plane's bulk copies never arrived");
     return TLM_OK;
 }
 

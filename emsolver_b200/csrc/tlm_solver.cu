@@ -794,8 +794,12 @@ template <class S> tlm_status launchStep(tlm_solver *h, int n, int i, long long 
 
 // The kernel shapes of two-step passes: wide columns first (they measured 4 %
 // faster per plane than the second's where both fit a grid equally), then
-// taller ones, which leave fewer lanes idle on grids the first cuts badly.
-using PairLayouts = std::tuple<tlmk::PairLayout<50, 10, 3, 1>, tlmk::PairLayout<34, 15, 3, 1>>;
+// taller ones, which leave fewer lanes idle on grids the first cuts badly, and
+// two for grids that one column of at most 40 or 16 nodes covers in x (of the
+// tallest boxes only two stages fit).
+using PairLayouts = std::tuple<tlmk::PairLayout<50, 10, 3, 1>, tlmk::PairLayout<34, 15, 3, 1>,
+                               tlmk::PairLayout<22, 23, 3, 1>, tlmk::PairLayout<10, 51, 2, 1>>;
+constexpr int kNarrowLayouts = 2;  // from this one on
 template <int I = 0, class F> void withPairLayout(int layout, F &&f)
 {
     if constexpr (I < (int)std::tuple_size<PairLayouts>::value)
@@ -809,13 +813,14 @@ template <int I = 0, class F> void withPairLayout(int layout, F &&f)
 
 // The columns with the least cost: blocks run one per SM and every plane of
 // one costs about the same, so a pass takes waves x planes per block (two of
-// them first-step planes of the neighbouring ranges).
-void choosePairShape(int ny, int nz, int px, int sms, tlmk::PairShape &best, int &layout)
+// them first-step planes of the neighbouring ranges). Returns that cost.
+long long choosePairShape(int ny, int nz, int px, int sms, tlmk::PairShape &best, int &layout)
 {
     long long bestCost = -1;
     for (int l = 0; l < (int)std::tuple_size<PairLayouts>::value; ++l)
         withPairLayout(l, [&](auto L) {
             using Layout = decltype(L);
+            if (l >= kNarrowLayouts && px > Layout::maxTX) return;
             const int ntx = (px + Layout::maxTX - 1) / Layout::maxTX;
             const int TX = ((px + ntx - 1) / ntx + 3) / 4 * 4;
             const int nty0 = (ny + Layout::maxTY - 1) / Layout::maxTY;
@@ -833,6 +838,24 @@ void choosePairShape(int ny, int nz, int px, int sms, tlmk::PairShape &best, int
                 }
             }
         });
+    return bestCost;
+}
+
+// Whether a pass of that cost takes less time than two single steps, on a grid
+// of `nodes` padded nodes of whose tiles the share `stubs` holds stub-loaded
+// nodes. In microseconds on a B200, from 45 shapes of 1.05 to 38 M nodes, air and
+// with dielectrics: a step of a pass takes 0.9 per plane of its cost and three
+// planes' worth per wave, 0.4 more where stubs hold the wave up (the only wave
+// waits for its slowest block, of several they make up their share); a single
+// step takes 8 (10 with stubs) and 15.1 (16.4) per million nodes. Columns that leave
+// most of a block idle, and few planes, for which the model does not hold, lose:
+// 8x400x400 air 77 us per step against 28 in single steps, 24x24x2000 with
+// dielectrics 38 against 25, 1000x1000x2 83 against 62, 500x500x5 36 against 32.
+bool pairPays(const tlmk::PairShape &g, long long cost, int nz, long long nodes, double stubs, int sms)
+{
+    const double waves = (double)(((long long)g.ntx * g.nty * g.nchunk + sms - 1) / sms), m = (double)nodes * 1e-6;
+    const double plane = 0.9 + (stubs > 0.0 ? 0.4 * (stubs + (1.0 - stubs) / waves) : 0.0);
+    return nz >= 10 && plane * ((double)cost + 3.0 * waves) <= (stubs > 0.0 ? 10.0 + 16.4 * m : 8.0 + 15.1 * m);
 }
 
 } // namespace tlmi
@@ -869,15 +892,18 @@ static tlm_status planPair(tlm_solver *h)
 {
     TensorMapEncoder encode = tensorMapEncoder();
     if (!encode) return TLM_OK;
+    int sms = 0;
+    TLM_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    auto plan = std::make_shared<PairPlan>();
+    const long long cost = choosePairShape(h->ny, h->nz, h->px, sms, plan->sh, plan->layout);
+    const tlmk::PairShape &g = plan->sh;
+    long long stubTiles = 0;
+    for (uint8_t f : h->tileFlagsHost) stubTiles += (f & tlmk::kTileDiel) != 0;
+    if (!pairPays(g, cost, h->nz, h->P, (double)stubTiles / h->nblocks, sms)) return TLM_OK;
     {
         const size_t need = (h->dStub ? 3 : 0) * (size_t)h->P * sizeof(float) + (size_t)(h->P / 2) * 12;
         if (!poolCovers(h->device, need) && poolAvailable(h->device) < need + ((size_t)256 << 20)) return TLM_OK;
     }
-    int sms = 0;
-    TLM_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    auto plan = std::make_shared<PairPlan>();
-    choosePairShape(h->ny, h->nz, h->px, sms, plan->sh, plan->layout);
-    const tlmk::PairShape &g = plan->sh;
     // the kernel's lane offsets within a plane are 32-bit byte offsets
     if ((long long)h->px * h->ny > (1LL << 28)) return TLM_OK;
     tlm_status st = TLM_OK;

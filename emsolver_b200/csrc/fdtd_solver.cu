@@ -1449,11 +1449,13 @@ void chooseFused(fdtd_solver *h, int sms)
             for (int rows = rows0; rows < rows0 + 6 && rows <= ny; ++rows)
             {
                 const int TY = (ny + rows - 1) / rows, nty = (ny + TY - 1) / TY;
-                for (int c = 1; c <= std::max(1, nz / 2); ++c)
+                // (of the counts of ranges with the same planes per range the smallest)
+                for (int c = 1, p = nz; c <= std::max(1, nz / 2); c = p > 1 ? (nz + p - 2) / (p - 1) : nz + 1)
                 {
+                    p = (nz + c - 1) / c;
                     const long long slots = (long long)sms * Layout::kMinBlocks;
                     const long long waves = ((long long)ntx * nty * c + slots - 1) / slots;
-                    const long long cost = waves * ((nz + c - 1) / c + (c > 1 ? 1 : 0)) *
+                    const long long cost = waves * (p + (c > 1 ? 1 : 0)) *
                                            (Layout::kThreads * Layout::kMinBlocks);
                     if (best >= 0 && cost >= best) continue;
                     best = cost;

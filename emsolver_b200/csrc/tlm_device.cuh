@@ -25,6 +25,13 @@
 namespace tlmk {
 
 constexpr int kBlock = 256;  // threads per block of the step kernel
+
+// The columns of a grid in passes of two steps: TX x TY nodes each, nchunk ranges of planes.
+struct PairShape
+{
+    int TX, TY, ntx, nty, nchunk;
+};
+
 constexpr int kPadX = 8;     // row pitch multiple (every vector width divides it)
 
 enum : uint8_t { kAir = 0, kPec = 1, kDiel0 = 2 };

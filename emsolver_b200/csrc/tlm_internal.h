@@ -311,6 +311,8 @@ struct tlm_solver
     // pass writes (swapped with dStub after every pass)
     std::shared_ptr<tlmi::PairPlan> pair;
     bool pairTried = false;
+    int pairFrom = 0, pairLayout = 0;    // steps from which the plan pays (0: not worked out), its kernel shape
+    tlmk::PairShape pairShape{};         // and columns
     size_t pairBytes = 0;                // device bytes of the plan
     bool planning = false;               // allocating for it
     bool noPair = false;                 // the server's budget has no room for it

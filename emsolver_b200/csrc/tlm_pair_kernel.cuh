@@ -54,12 +54,6 @@ namespace tlmk {
 // of the energy steps, so that one test sends a plane past all the rare work.
 enum : unsigned { kPairPec = 1, kPairSpec = 2, kPairDiel = 4, kPairWallZ = 8, kPairEnergy0 = 16, kPairEnergy1 = 32 };
 
-// The columns of a grid: TX x TY nodes each, nchunk ranges of planes.
-struct PairShape
-{
-    int TX, TY, ntx, nty, nchunk;
-};
-
 // A kernel shape: W pairs x H rows of threads cover the grown column (x0-2 ..
 // x0+TX+1, y0-1 .. y0+TY), for TX <= 2W-4 and TY <= H-2; a stage row holds the
 // W2 nodes from x0-4 on (16-byte aligned box starts). The strides are

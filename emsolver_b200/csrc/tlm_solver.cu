@@ -101,6 +101,7 @@ void dropPair(tlm_solver *h)
     std::lock_guard<std::recursive_timed_mutex> lk(h->lender.busy);
     h->pair.reset();
     h->pairTried = false;
+    h->pairFrom = 0;
     devFree(h, h->dPairFlags);
     devFree(h, h->dPairWord);
     devFree(h, h->dSpecRow);
@@ -827,10 +828,12 @@ long long choosePairShape(int ny, int nz, int px, int sms, tlmk::PairShape &best
             for (int rows = nty0; rows < nty0 + 6 && rows <= ny; ++rows)
             {
                 const int TY = (ny + rows - 1) / rows, nty = (ny + TY - 1) / TY;
-                for (int c = 1; c <= std::max(1, nz / 4); ++c)
+                // (of the counts of ranges with the same planes per range the smallest)
+                for (int c = 1, p = nz; c <= std::max(1, nz / 4); c = p > 1 ? (nz + p - 2) / (p - 1) : nz + 1)
                 {
+                    p = (nz + c - 1) / c;
                     const long long waves = ((long long)ntx * nty * c + sms - 1) / sms;
-                    const long long cost = waves * ((nz + c - 1) / c + (c > 2 ? 2 : c - 1) + 1);
+                    const long long cost = waves * (p + (c > 2 ? 2 : c - 1) + 1);
                     if (bestCost >= 0 && cost >= bestCost) continue;
                     bestCost = cost;
                     best = tlmk::PairShape{ TX, TY, ntx, nty, c };
@@ -841,9 +844,9 @@ long long choosePairShape(int ny, int nz, int px, int sms, tlmk::PairShape &best
     return bestCost;
 }
 
-// Whether a pass of that cost takes less time than two single steps, on a grid
+// What a pass of that cost saves per step over single steps, on a grid
 // of `nodes` padded nodes of whose tiles the share `stubs` holds stub-loaded
-// nodes. In microseconds on a B200, from 45 shapes of 1.05 to 38 M nodes, air and
+// nodes (not positive: nothing). In microseconds on a B200, from 45 shapes of 1.05 to 38 M nodes, air and
 // with dielectrics: a step of a pass takes 0.9 per plane of its cost and three
 // planes' worth per wave, 0.4 more where stubs hold the wave up (the only wave
 // waits for its slowest block, of several they make up their share); a single
@@ -851,11 +854,12 @@ long long choosePairShape(int ny, int nz, int px, int sms, tlmk::PairShape &best
 // most of a block idle, and few planes, for which the model does not hold, lose:
 // 8x400x400 air 77 us per step against 28 in single steps, 24x24x2000 with
 // dielectrics 38 against 25, 1000x1000x2 83 against 62, 500x500x5 36 against 32.
-bool pairPays(const tlmk::PairShape &g, long long cost, int nz, long long nodes, double stubs, int sms)
+double pairSaving(const tlmk::PairShape &g, long long cost, int nz, long long nodes, double stubs, int sms)
 {
+    if (nz < 10) return 0.0;
     const double waves = (double)(((long long)g.ntx * g.nty * g.nchunk + sms - 1) / sms), m = (double)nodes * 1e-6;
     const double plane = 0.9 + (stubs > 0.0 ? 0.4 * (stubs + (1.0 - stubs) / waves) : 0.0);
-    return nz >= 10 && plane * ((double)cost + 3.0 * waves) <= (stubs > 0.0 ? 10.0 + 16.4 * m : 8.0 + 15.1 * m);
+    return (stubs > 0.0 ? 10.0 + 16.4 * m : 8.0 + 15.1 * m) - plane * ((double)cost + 3.0 * waves);
 }
 
 } // namespace tlmi
@@ -886,20 +890,33 @@ TensorMapEncoder tensorMapEncoder()
     return fn;
 }
 
+// The number of steps that saves as much as making the plan of the handle's
+// two-step passes takes (80 us at 104^3, 160 at 192^3); INT_MAX: never. Worked out
+// once per prepare, with the columns.
+int pairPaysFrom(tlm_solver *h)
+{
+    if (h->pairFrom > 0) return h->pairFrom;
+    h->pairFrom = INT_MAX;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) return h->pairFrom;
+    const long long cost = choosePairShape(h->ny, h->nz, h->px, sms, h->pairShape, h->pairLayout);
+    long long stubTiles = 0;
+    for (uint8_t f : h->tileFlagsHost) stubTiles += (f & tlmk::kTileDiel) != 0;
+    const double saving = pairSaving(h->pairShape, cost, h->nz, h->P, (double)stubTiles / h->nblocks, sms);
+    if (saving > 0.0) h->pairFrom = (int)std::min(1e9, 2.0 + (60.0 + 14e-6 * (double)h->P) / saving);
+    return h->pairFrom;
+}
+
 // Plan the two-step passes of a handle (h->pair stays null where they are not
 // possible).
 static tlm_status planPair(tlm_solver *h)
 {
     TensorMapEncoder encode = tensorMapEncoder();
-    if (!encode) return TLM_OK;
-    int sms = 0;
-    TLM_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    if (!encode || pairPaysFrom(h) == INT_MAX) return TLM_OK;
     auto plan = std::make_shared<PairPlan>();
-    const long long cost = choosePairShape(h->ny, h->nz, h->px, sms, plan->sh, plan->layout);
+    plan->sh = h->pairShape;
+    plan->layout = h->pairLayout;
     const tlmk::PairShape &g = plan->sh;
-    long long stubTiles = 0;
-    for (uint8_t f : h->tileFlagsHost) stubTiles += (f & tlmk::kTileDiel) != 0;
-    if (!pairPays(g, cost, h->nz, h->P, (double)stubTiles / h->nblocks, sms)) return TLM_OK;
     {
         const size_t need = (h->dStub ? 3 : 0) * (size_t)h->P * sizeof(float) + (size_t)(h->P / 2) * 12;
         if (!poolCovers(h->device, need) && poolAvailable(h->device) < need + ((size_t)256 << 20)) return TLM_OK;
@@ -1276,7 +1293,8 @@ tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stoppe
             }
             if (i + 1 < w && pairAllowed(h))
             {
-                TLM_TRY(ensurePair(h));
+                // (steps from 0 on: a host that steps little by little plans in the end)
+                if (!h->pairTried && base + remaining >= pairPaysFrom(h)) TLM_TRY(ensurePair(h));
                 if (h->pair)
                 {
                     TLM_TRY(launchPair(h, n, i, eFirst));

@@ -19,7 +19,8 @@
 // sources; without room for a second field buffer they run in place,
 // one sweep for H and one for E.
 // Fields: one plane set per component, all six with the same pitch (cell
-// (i, j, k) of every component at (k*(ny+1) + j)*px + i; entries that a
+// (i, j, k) of every component at (k*(ny+1) + j)*px + i, rows padded for fused
+// passes only; entries that a
 // component does not have stay zero). All arithmetic is FP32 in the
 // reference's operation order (the library is compiled with --fmad=false),
 // hence bitwise results.
@@ -48,7 +49,7 @@ namespace fdk {
 struct Dims
 {
     int nx, ny, nz;
-    int px;  // row pitch: nx + 1 rounded up to 4
+    int px;  // row pitch: nx + 1, rounded up to 4 for fused passes
     __host__ __device__ long long at(int i, int j, int k) const { return ((long long)k * (ny + 1) + j) * px + i; }
     __host__ __device__ long long iEx(int i, int j, int k) const { return at(i, j, k); }
     __host__ __device__ long long iEy(int i, int j, int k) const { return at(i, j, k); }
@@ -57,7 +58,8 @@ struct Dims
     __host__ __device__ long long iHy(int i, int j, int k) const { return at(i, j, k); }
     __host__ __device__ long long iHz(int i, int j, int k) const { return at(i, j, k); }
     // 32-bit form for the in-place sweeps: setup refuses grids whose
-    // (nx+1)(ny+1)(nz+1) index box reaches 2^31, and the pitch adds at most a third.
+    // (nx+1)(ny+1)(nz+1) index box reaches 2^31, and the pitch adds at most
+    // three fifths (8 for 5).
     __device__ unsigned q(int i, int j, int k) const
     {
         return ((unsigned)k * (unsigned)(ny + 1) + (unsigned)j) * (unsigned)px + (unsigned)i;
@@ -1434,8 +1436,9 @@ template <int I = 0, class F> void withFusedLayout(int layout, F &&f)
 }
 
 // The columns of fused passes with the least cost: waves of resident blocks
-// times planes (one of them the ring's plane below) times a block's threads.
-void chooseFused(fdtd_solver *h, int sms)
+// times planes (one of them the ring's plane below) times the threads of an SM's
+// blocks. Returns it.
+long long chooseFused(fdtd_solver *h, int sms)
 {
     const fdk::Dims &d = h->d;
     long long best = -1;
@@ -1468,6 +1471,21 @@ void chooseFused(fdtd_solver *h, int sms)
                 }
             }
         });
+    return best;
+}
+
+// Whether a fused pass of that cost takes less time than the in-place sweeps.
+// Microseconds on a B200, from 51 shapes of 27 to 8 M cells: a pass takes 13
+// with its tail, 1.9 per 1024 of its cost (2.2 with dielectrics), and 5 per
+// million edges of the x faces, whose values lie a row apart (30 where the fields
+// exceed L2); the sweeps take 27 and 10 per million cells, from about 1.3 M on 18
+// and 17. Columns that leave most of a block idle lose: 4x500x500 air 83 us
+// fused, 47 in place, 2x2x8000 32 and 21, 8x600x600 with dielectrics 141 and 91.
+bool fusedPays(const fdk::Dims &d, long long cost, bool diel)
+{
+    const double m = (double)(d.nx + 1) * (d.ny + 1) * (d.nz + 1) * 1e-6, faces = 4.0 * d.ny * d.nz * 1e-6;
+    const double pass = 13.0 + (diel ? 2.2 : 1.9) * (double)cost / 1024.0 + (m > 2.5 ? 30.0 : 5.0) * faces;
+    return pass <= std::max(27.0 + 10.0 * m, 18.0 + 17.0 * m);
 }
 
 // Tensor maps of the fused pass's boxes and the kernel's shared memory.
@@ -1528,9 +1546,6 @@ tlm_status allocFused(fdtd_solver *h)
     FD_TRY(alloc(h, &h->dBuf[1], field));
     if (reinterpret_cast<uintptr_t>(h->dBuf[1]) & 15) return h->fail(TLM_ECUDA, "field allocation not 16-byte aligned");
     FD_CU(h, cudaMemsetAsync(h->dBuf[1], 0, field, h->stream));
-    int sms = 0;
-    FD_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    chooseFused(h, sms);
     h->fault = faultWords().take();
     if (!h->fault) return h->fail(TLM_ENOMEM, "no fault word");
     FD_TRY(fusedMaps(h));
@@ -1832,31 +1847,47 @@ tlm_status fdtd_setup(fdtd_handle h, const tlm_grid *grid, const uint8_t *mat, s
     h->cfg = *cfg;
     h->mat.swap(hostMat);
     h->table.assign(table, table + n_table);
+    h->haveDiel = maxId >= TLM_MAT_DIEL0;
     h->d = fdk::Dims{ grid->nx, grid->ny, grid->nz, (grid->nx + 4) / 4 * 4 };
     const fdk::Dims &d = h->d;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
+    // fused passes where they pay (their lane offsets within a plane are 32-bit),
+    // with rows padded for them; no_staging asks for the in-place sweeps on the
+    // same rows
+    int sms = 0;
+    FD_CU(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    bool fused = (long long)d.px * (ny + 1) < (1LL << 30) && tlmi::tensorMapEncoder() != nullptr &&
+                 fusedPays(d, chooseFused(h, sms), h->haveDiel);
+    if (!fused) h->d.px = nx + 1;
+    fused = fused && !cfg->no_staging;
     h->dt = tlmh::fdtd_dt(grid->dl);
     h->cMur = tlmh::fdtd_cmur(h->dt, grid->dl);
     h->cb0 = tlmh::fdtd_cb0(h->dt, grid->dl);
     h->ch = tlmh::fdtd_ch(h->dt, grid->dl);
-    h->haveDiel = maxId >= TLM_MAT_DIEL0;
     h->len[0] = (long long)nx * (ny + 1) * (nz + 1);
     h->len[1] = (long long)(nx + 1) * ny * (nz + 1);
     h->len[2] = (long long)(nx + 1) * (ny + 1) * nz;
     h->len[3] = (long long)(nx + 1) * ny * nz;
     h->len[4] = (long long)nx * (ny + 1) * nz;
     h->len[5] = (long long)nx * ny * (nz + 1);
-    h->P = (long long)d.px * (ny + 1) * (nz + 1);
+    // (components start on 16 bytes)
+    auto planeSet = [&] { return ((long long)d.px * (ny + 1) * (nz + 1) + 3) / 4 * 4; };
+    h->P = planeSet();
     h->cur = 0;
-    const size_t field = fieldBytes(h), classes = (size_t)h->P * 4, mixed = h->haveDiel ? 6 * (size_t)h->P * 4 : 0;
-    const size_t need = field + classes + mixed, spare = (size_t)256 << 20;
+    // fields, edge classes, coefficients of mixed edges
+    const size_t spare = (size_t)256 << 20;
+    auto bytes = [&] { return (size_t)h->P * 4 * (h->haveDiel ? 13 : 7); };
     size_t avail = tlmi::poolAvailable(h->device);
+    // a second field buffer for fused passes where it fits
+    if (fused && bytes() + fieldBytes(h) + spare > avail)
+    {
+        fused = false;
+        h->d.px = nx + 1;
+        h->P = planeSet();
+    }
+    const size_t need = bytes(), field = fieldBytes(h), classes = (size_t)h->P * 4;
     if (need + spare > avail && tlmi::reclaim(h->device)) avail = tlmi::poolAvailable(h->device);
     if (need + spare > avail) return h->fail(TLM_ENOMEM, "grid needs " + std::to_string(need >> 20) + " MiB of HBM");
-    // a second field buffer for fused passes where it fits (their lane offsets
-    // within a plane are 32-bit); no_staging asks for the in-place sweeps
-    const bool fused = need + field + spare <= avail && !cfg->no_staging && (long long)d.px * (ny + 1) < (1LL << 30) &&
-                       tlmi::tensorMapEncoder() != nullptr;
     FD_TRY(alloc(h, &h->dBuf[0], field));
     if (reinterpret_cast<uintptr_t>(h->dBuf[0]) & 15)  // vector loads
         return h->fail(TLM_ECUDA, "field allocation not 16-byte aligned");

@@ -195,6 +195,8 @@ struct PairPlan;
 // 1.12 M nodes, 23-27 us per step against 25-27 with single steps; at 96^3 the
 // two are even, at 88^3 14.2 against 13.3 us).
 constexpr long long kPairMinNodes = 1LL << 20;
+// Resident windows that a call which waits for its steps keeps on the device.
+constexpr int kResidentAhead = 4;
 inline bool pairStorage(int storage, long long P) { return storage == TLM_STORE_F32 && P >= kPairMinNodes; }
 
 // A handle's share in the device memory that handles hold for speed alone and
@@ -328,6 +330,7 @@ struct tlm_solver
     int resBy = 0, resBz = 0, resPairs = 0;
     void *dResPack = nullptr;
     unsigned resBase = 0;
+    cudaEvent_t resDone[tlmi::kResidentAhead] = {};  // ends of the last windows that a waiting call launched
     double *dEpair = nullptr;
     std::vector<uint8_t> tileFlagsHost;
     void *dSamples = nullptr;

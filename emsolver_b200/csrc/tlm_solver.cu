@@ -1258,13 +1258,31 @@ template <class R> tlm_status launchEpilogue(tlm_solver *h, long long base, int 
     return h->cuda(cudaGetLastError(), "windowEpilogue launch");
 }
 
-// Enqueue n steps in windows of h->window; optionally stop early.
-tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stopped)
+// Wait until at most kResidentAhead - 1 of the resident windows that this call
+// launched are left on the device, then note one more. Resident launches of a
+// device follow one another (ResidentOrder), so that windows queued without end
+// would hold up every other handle's: a call that waits for its steps anyway
+// keeps the queue short.
+tlm_status boundResident(tlm_solver *h, long long window)
+{
+    cudaEvent_t &ev = h->resDone[window % kResidentAhead];
+    if (!ev)
+        TLM_CU(h, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    else if (window >= kResidentAhead)
+        TLM_CU(h, cudaEventSynchronize(ev));
+    TLM_CU(h, cudaEventRecord(ev, h->stream));
+    return TLM_OK;
+}
+
+// Enqueue n steps in windows of h->window; optionally stop early. `waits`: the
+// caller waits for the steps.
+tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stopped, bool waits = false)
 {
     if (stopped) *stopped = false;
     std::lock_guard<std::recursive_timed_mutex> lk(h->lender.busy);
     TLM_TRY(prepare(h));
     int remaining = nsteps;
+    long long residentWindows = 0;
     while (remaining > 0)
     {
         if (honourStop && h->stopFlag.load())
@@ -1277,6 +1295,7 @@ tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stoppe
         TLM_TRY(ensureRecords(h, base + w));
         const long long eFirst = (base + 15) / 16 * 16;
         const int nE = eFirst < base + w ? (int)((base + w - 1 - eFirst) / 16 + 1) : 0;
+        bool resident = false;
         for (int i = 0; i < w; ++i)
         {
             const int n = (int)(base + i);
@@ -1287,6 +1306,7 @@ tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stoppe
                 {
                     const int steps = std::min(w - i, tlmk::kResidentSteps);
                     TLM_TRY(launchResident(h, n, i, steps, eFirst));
+                    resident = true;
                     i += steps - 1;
                     continue;
                 }
@@ -1318,6 +1338,7 @@ tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stoppe
         h->curStep += w;
         ++h->recVersion;
         remaining -= w;
+        if (waits && resident && nsteps > kResidentAhead * h->window) TLM_TRY(boundResident(h, residentWindows++));
         if (honourStop)
         {
             // keep at most one window in flight so that a stop request or a
@@ -1729,6 +1750,8 @@ tlm_status tlm_destroy(tlm_handle h)
     if (h->dElatest) cudaFreeAsync(h->dElatest, h->stream);
     if (h->dFault) cudaFreeAsync(h->dFault, h->stream);
     for (cudaEvent_t ev : h->evs) cudaEventDestroy(ev);
+    for (cudaEvent_t ev : h->resDone)
+        if (ev) cudaEventDestroy(ev);
     if (h->side)
     {
         cudaStreamSynchronize(h->side);
@@ -2074,7 +2097,7 @@ tlm_status tlmi::chooseScale(tlm_solver *h)
 extern "C" {
 
 
-tlm_status tlm_step_async(tlm_handle h, int n_steps)
+static tlm_status stepHandle(tlm_solver *h, int n_steps, bool waits)
 {
     TLM_TRY(checkReady(h));
     if (h->batch) return h->fail(TLM_ESTATE, "the handle is attached to a batch: step the batch");
@@ -2083,8 +2106,10 @@ tlm_status tlm_step_async(tlm_handle h, int n_steps)
         return h->fail(TLM_ESTATE, "slab steps are open: end them and call tlm_slab_flush first");
     DeviceGuard dg(h->device);
     if (h->curStep == 0 && !h->prepared) TLM_TRY(chooseScale(h));
-    return enqueueSteps(h, n_steps, false, nullptr);
+    return enqueueSteps(h, n_steps, false, nullptr, waits);
 }
+
+tlm_status tlm_step_async(tlm_handle h, int n_steps) { return stepHandle(h, n_steps, false); }
 
 tlm_status tlm_sync(tlm_handle h)
 {
@@ -2095,7 +2120,7 @@ tlm_status tlm_sync(tlm_handle h)
 
 tlm_status tlm_step(tlm_handle h, int n_steps)
 {
-    TLM_TRY(tlm_step_async(h, n_steps));
+    TLM_TRY(stepHandle(h, n_steps, true));
     DeviceGuard dg(h->device);
     return syncState(h);
 }

@@ -216,7 +216,10 @@ TLM_API tlm_status tlm_set_port_dft(tlm_handle h, const double *freqs_hz, int n_
 TLM_API tlm_status tlm_step(tlm_handle h, int n_steps);
 
 /* Same, without waiting: the work is queued on the handle's stream.
- * Results are visible after tlm_sync (or any getter, which syncs). */
+ * Results are visible after tlm_sync (or any getter, which syncs). FP32 grids
+ * that fit the card's shared memory take all of it for a launch window, and the
+ * windows of a device's handles run in the order they were queued; tlm_step
+ * queues a few windows ahead, this call all of them. */
 TLM_API tlm_status tlm_step_async(tlm_handle h, int n_steps);
 TLM_API tlm_status tlm_sync(tlm_handle h);
 

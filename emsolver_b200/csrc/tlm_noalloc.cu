@@ -14,7 +14,7 @@
 // buffers), and the last block to finish adds up the blocks' energies in a
 // fixed order. The only scratch, an FP64 partial per block and the count of
 // finished blocks, 16 slots of them, lives in the file-scope arrays below, a fixed
-// 74 KiB of device memory that every GPU which loads this library holds until the
+// 296 KiB of device memory that every GPU which loads this library holds until the
 // process exits. Host code must not pass an array's name to a kernel (on the
 // host that name is a stand-in, not a device address); the device addresses
 // are looked up once per device with cudaGetSymbolAddress.
@@ -33,7 +33,8 @@ void tlmSetThreadError(const std::string &m);
 
 // The grid is limited to 67,108,864 padded nodes (2^25 pairs).
 constexpr long long kNoAllocMaxNodes = 67108864;
-constexpr int kNoAllocMaxBlocks = 148 * 4, kNoAllocSlots = 16;
+constexpr unsigned kNoAllocWave = 148 * 4;  // resident blocks
+constexpr int kNoAllocMaxBlocks = 4 * kNoAllocWave, kNoAllocSlots = 16;
 static __device__ __align__(256) double g_noallocPartials[kNoAllocSlots * kNoAllocMaxBlocks];
 static __device__ __align__(256) unsigned long long g_noallocDone[kNoAllocSlots];
 constexpr int kNoAllocTable = 256 - tlmk::kDiel0;
@@ -373,8 +374,16 @@ tlm_status tlm_step_planes_noalloc(const float *in_planes, float *out_planes, fl
             return noallocFail(TLM_ECUDA, std::string("no-allocation step set-up: ") + cudaGetErrorString(e));
     }
     a.fault = sc.fault;
-    // four resident blocks per SM walk over the tiles of large grids
-    const unsigned blocks = std::min((a.npairs + 255u) / 256u, (unsigned)kNoAllocMaxBlocks);
+    // Blocks that walk over several tiles of 256 pairs leave fewer partials to
+    // add up, but nothing of their next tile is in flight while they finish one:
+    // with an energy the grid is a wave of blocks per 4096 tiles, at most four,
+    // without one a block per tile beyond two waves. One wave for all sizes took
+    // 576 us for incident planes of 320^3 nodes without an energy, 574 with one;
+    // now 469 and 508 (128^3: 38 and 41, now 36 and 41).
+    const unsigned tiles = (a.npairs + 255u) / 256u;
+    const unsigned most = energy_out ? kNoAllocWave * std::min(std::max(tiles / 4096u, 1u), 4u)
+                          : tiles <= 2 * kNoAllocWave ? kNoAllocWave : tiles;
+    const unsigned blocks = std::min(tiles, most);
     if (input_is_incident)
     {
         if (stubs) planesStepKernel<true, true><<<blocks, 256, 0, s>>>(a);

@@ -560,7 +560,7 @@ TLM_API tlm_status tlm_get_halo_stream(tlm_handle h, void **stream);
  * Work is queued on `stream` (a cudaStream_t, NULL = default stream).
  *
  * Limits and sharing: its only scratch, one FP64 energy partial per thread
- * block and a count of finished blocks, is 16 slots in a fixed 74 KiB of static device
+ * block and a count of finished blocks, is 16 slots in a fixed 296 KiB of static device
  * arrays that every GPU loading this library holds until the process exits;
  * grids above 67,108,864 padded nodes are rejected with TLM_EINVAL. The
  * first call on a device looks up those arrays' device addresses

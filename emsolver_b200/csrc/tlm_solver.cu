@@ -1302,7 +1302,10 @@ tlm_status enqueueSteps(tlm_solver *h, int nsteps, bool honourStop, bool *stoppe
             if (i + 1 < w && residentAllowed(h))
             {
                 TLM_TRY(ensureResident(h));
-                if (h->resBy > 0)
+                // (loading and storing two pairs per thread takes as long as about
+                // three single steps: two steps of 61x53x47 per call 62 us
+                // resident, 54 in the single kernel; four 67 and 71)
+                if (h->resBy > 0 && w - i >= (h->resPairs > tlmk::kResidentThreads ? 4 : 2))
                 {
                     const int steps = std::min(w - i, tlmk::kResidentSteps);
                     TLM_TRY(launchResident(h, n, i, steps, eFirst));

@@ -293,22 +293,6 @@ __global__ void stubsToAos(const R *__restrict__ stub, long long P, int nx, int 
     }
 }
 
-template <class R>
-__global__ void aosToStubs(const R *__restrict__ in, long long P, int nx, int ny, int nz, int px,
-                           R *__restrict__ stub)
-{
-    for (long long node = blockIdx.x * (long long)blockDim.x + threadIdx.x; node < P;
-         node += (long long)gridDim.x * blockDim.x)
-    {
-        const int i = (int)(node % px);
-        const long long r = node / px;
-        const int j = (int)(r % ny), k = (int)(r / ny);
-        const bool real = i < nx && k < nz;
-        const long long c = ((long long)k * ny + j) * nx + i;
-        for (int s = 0; s < 3; ++s) stub[s * P + node] = real ? in[c * 3 + s] : R(0);
-    }
-}
-
 // Material map in the reference's cell order -> the padded layout (row pitch
 // px, padding columns PEC), one padded node per thread.
 static __global__ void padMaterial(const uint8_t *__restrict__ raw, int nx, int px, long long rows,

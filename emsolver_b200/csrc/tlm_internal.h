@@ -191,9 +191,9 @@ struct SurfaceState
 // The plan of two-step passes (tlm_pair_kernel.cuh; defined in tlm_solver.cu).
 struct PairPlan;
 
-// Two-step passes serve FP32 grids from this many padded nodes on (at 104^3,
-// 1.12 M nodes, 23-27 us per step against 25-27 with single steps; at 96^3 the
-// two are even, at 88^3 14.2 against 13.3 us).
+// Two-step passes serve FP32 grids from this many padded nodes on, where they
+// pay (104^3, 1.12 M nodes: 20 us per step in air and 26 with dielectrics against
+// 26 and 31 in single steps; at 96^3 the two were even, at 88^3 14.2 against 13.3).
 constexpr long long kPairMinNodes = 1LL << 20;
 // Resident windows that a call which waits for its steps keeps on the device.
 constexpr int kResidentAhead = 4;

@@ -122,8 +122,7 @@ __device__ void incidentAt(const SurfaceArgs<S> &a, long long node, int i, int j
     }
 }
 
-// (a face node below 2^32 takes 32-bit divisions; every grid of 16-bit pulses
-// or wider that fits the card is below)
+// (32-bit divisions for nodes below 2^32, as on every grid that fits 180 GB)
 __device__ __forceinline__ void cellOfNode(long long node, int px, int ny, int *i, int *j, int *k)
 {
     if (node >> 32)

@@ -448,10 +448,15 @@ void buildFaceLists(int nx, int ny, int nz, const float origin[3], float dl, con
     const int dims[3] = { nx, ny, nz };
     for (int k = 0; k < nz; ++k)
         for (int j = 0; j < ny; ++j)
-            for (int i = 0; i < nx; ++i)
+        {
+            // the row's PEC cells by memchr: a loop over its bytes took 300 or
+            // 440 us for 1 M cells, by where the linker put it
+            const uint8_t *row = mat + ((size_t)k * ny + j) * nx;
+            for (const uint8_t *m = row; (m = static_cast<const uint8_t *>(std::memchr(m, tlmk::kPec, row + nx - m)));
+                 ++m)
             {
-                const size_t c = ((size_t)k * ny + j) * nx + i;
-                if (mat[c] != tlmk::kPec) continue;
+                const int i = (int)(m - row);
+                const size_t c = m - mat;
                 const int co[3] = { i, j, k };
                 for (int a = 0; a < 3; ++a)
                     for (int sd = -1; sd <= 1; sd += 2)
@@ -469,6 +474,7 @@ void buildFaceLists(int nx, int ny, int nz, const float origin[3], float dl, con
                         s.jsCenter.insert(s.jsCenter.end(), cc, cc + 3);
                     }
             }
+        }
     const int o = huyOffset;
     if (o < 2 || 2 * o + 2 >= nx || 2 * o + 2 >= ny || 2 * o + 2 >= nz) return;
     const float half[3] = { ((float)nx * dl) * 0.5f, ((float)ny * dl) * 0.5f, ((float)nz * dl) * 0.5f };

@@ -1193,9 +1193,8 @@ class FaultWords
     unsigned *take()
     {
         std::lock_guard<std::mutex> lk(mu_);
-        if (!page_ && !tried_)
+        if (!page_)
         {
-            tried_ = true;
             void *p = nullptr;
             if (cudaHostAlloc(&p, kWords * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
                 cudaGetLastError();
@@ -1218,7 +1217,6 @@ class FaultWords
   private:
     static constexpr int kWords = 4096;
     std::mutex mu_;
-    bool tried_ = false;
     unsigned *page_ = nullptr;
     std::vector<unsigned *> free_;
 };

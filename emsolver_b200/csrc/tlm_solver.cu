@@ -1120,9 +1120,14 @@ tlm_status ensureResident(tlm_solver *h)
     // two parities of two directions per axis, zero: no step has the number 0
     const size_t packs = 4 * (size_t)hx * ((size_t)gy * h->nz + (size_t)gz * h->ny) * sizeof(tlmk::ResPacket);
     const size_t share = (size_t)(tlmk::kResidentSteps / 16 + 1) * (h->P / 2) * sizeof(double);
-    if (e != cudaSuccess || perSm < 1 || devAlloc(h, &h->dResPack, packs) != TLM_OK ||
-        devAlloc(h, &h->dEpair, share) != TLM_OK)
+    const std::string err = h->err;
+    h->planning = true;  // (no handle gives up a plan for this one)
+    const bool ok = e == cudaSuccess && perSm >= 1 && devAlloc(h, &h->dResPack, packs) == TLM_OK &&
+                    devAlloc(h, &h->dEpair, share) == TLM_OK;
+    h->planning = false;
+    if (!ok)
     {
+        h->err = err;
         cudaGetLastError();
         devFree(h, h->dResPack);
         h->resBy = 0;
